@@ -217,6 +217,20 @@ int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_val
                      uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
                      int tile_cols, int grid);
 
+/* The same over parts of segments (16 x 128 and 16 x 256 tiles), for plans with fewer
+ * segments than the GPU has room for.  12 uint32 each: row0, nrow, col0, ncol, w0, w1,
+ * part, tile, s0, s1 and two unused: windows [w0, w1), w0 < w1, of the segment [s0, s1),
+ * the parts of a segment covering it in order.  Each part takes the FP32 accumulator
+ * runs (of `fold` slots per lane) that begin in its windows, so the sums are those of
+ * the unsplit segment. */
+int phyloPairsLaunchParts(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
+                          uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
+                          uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,
+                          unsigned int num_windows, int window_shift, uintptr_t d_rowids,
+                          uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
+                          uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
+                          int tile_cols, int grid);
+
 /* Sums the partial blocks of each tile (4 uint32: row0, nrow, col0, ncol) into
  * d_out[rowid * ldc + colid] (double); `upper` 1 keeps pairs whose row position
  * is below the column position, 2 also the diagonal (row position == column
@@ -224,6 +238,12 @@ int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_val
 int phyloPairsReduce(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
                      int segments, int tile_rows, int tile_cols, uintptr_t d_rowids,
                      uintptr_t d_colids, uintptr_t d_out, long ldc, int upper, int mirror);
+
+/* The same for tiles whose partial blocks are counted per tile (8 uint32: row0, nrow,
+ * col0, ncol, first partial block, number of blocks, two unused). */
+int phyloPairsReduceParts(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
+                          int tile_rows, int tile_cols, uintptr_t d_rowids, uintptr_t d_colids,
+                          uintptr_t d_out, long ldc, int upper, int mirror);
 
 /* d_out[v * ldc + v] = sum of squares of vector v (the diagonal the
  * reference's run includes, phylogenetics_analysis/Main.java:196); d_part is

@@ -99,6 +99,11 @@ def _declare(L: ctypes.CDLL) -> None:
                                    c_uint, c_int, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_int,
                                    c_ptr, c_int, c_int, c_int]
     L.phyloPairsLaunch.restype = c_int
+    L.phyloPairsLaunchParts.argtypes = L.phyloPairsLaunch.argtypes
+    L.phyloPairsLaunchParts.restype = c_int
+    L.phyloPairsReduceParts.argtypes = [c_ptr, c_ptr, c_ptr, c_int, c_int, c_int, c_ptr, c_ptr,
+                                        c_ptr, c_long, c_int, c_int]
+    L.phyloPairsReduceParts.restype = c_int
     L.phyloPairsReduce.argtypes = [c_ptr, c_ptr, c_ptr, c_int, c_int, c_int, c_int, c_ptr, c_ptr,
                                    c_ptr, c_long, c_int, c_int]
     L.phyloPairsReduce.restype = c_int
@@ -149,7 +154,7 @@ EXPORTED = [
     "phyloBuildBatchSummaryBytes", "phyloBuildBatchEmit", "phyloBuildBatchNorms",
     "phyloBuildBatchCounts", "phyloBuildLaunchesPerBatch", "phyloWindowIndex",
     "phyloPairsPrepare", "phyloPairsSmemBytes", "phyloPairsThreads", "phyloPairsLaunch",
-    "phyloPairsReduce",
+    "phyloPairsLaunchParts", "phyloPairsReduce", "phyloPairsReduceParts",
     "phyloSelfDot", "phyloSelfDotPartBytes", "phyloKeyRankScratch", "phyloKeyRankBitmapBytes",
     "phyloKeyRanks", "phyloKeyRankIndex",
     "phyloCompareTileElements", "phyloComparePairsManyScratch",

@@ -11,8 +11,7 @@
 //     sub-list in every window.
 //   * A work item is 16 row vectors x up to 256 column vectors x a run of
 //     windows.  For each window the 16 row sub-lists are scattered into a
-//     shared-memory table D[key - r*W] of 80-byte records (16 row values +
-//     padding: the odd stride spreads random gathers over the banks; one extra
+//     shared-memory table D[key - r*W] of 64-byte records (16 row values; one extra
 //     zero record serves masked lanes).  The item's columns share the CTA's
 //     lanes evenly (two or four lanes per column); a column's lanes stream its
 //     sub-list in 16-byte groups through cp.async rings, and every entry (key, b)
@@ -31,50 +30,69 @@
 
 namespace phylo {
 
-// The row table D holds, for each key of the window, the 16 row values in one
-// 80-byte record (64 bytes of values + 16 bytes of padding).  The odd stride
-// (5 x 16 bytes) spreads the four 16-byte loads of random keys over all eight
-// 16-byte bank groups, and the four loads of a key are one base address plus
-// constant offsets.  One extra record (index W) stays zero for masked lanes.
-constexpr uint32_t D_STRIDE = 20;  // floats per key record
+// The row table holds, for each key of the window, the 16 row values in one 64-byte
+// record.  A lane reads a record as four 16-byte chunks in the order t ^ (lane & 3), so of
+// the eight lanes of a load phase only two can meet in a bank group: those with the same
+// order whose keys have the same parity.  (Padded 80-byte records, read in row order,
+// spread random keys over all eight bank groups and conflicted more: all pairs of 64
+// uniform proteomes of 1,500 proteins took 500 M load wavefronts, 282 M of them conflicts,
+// against 381 M and 163 M, and 2.55 ms against 2.10 with the packed FP32 FMAs and the
+// row scatter below.)  One extra record (index W) stays zero for masked lanes.
+constexpr uint32_t D_REC = 64;  // bytes per key record
 
-static size_t ap_ring_bytes(int threads);
-
-// float index of (key idx, row) in D
-__device__ __forceinline__ uint32_t d_slot(uint32_t idx, uint32_t row) {
-    return idx * D_STRIDE + row;
+// acc (two FP32 sums) += record values * b, each as __fmaf_rn
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t d, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(d), "l"(b));
+}
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
 }
 
-__device__ __forceinline__ void fma_entry(const float *__restrict__ D, uint32_t idx, float b,
-                                          float (&acc)[16]) {
-    const float4 *rowp = reinterpret_cast<const float4 *>(D + idx * D_STRIDE);
-    const float4 q0 = rowp[0], q1 = rowp[1], q2 = rowp[2], q3 = rowp[3];
-    acc[0] = __fmaf_rn(q0.x, b, acc[0]);
-    acc[1] = __fmaf_rn(q0.y, b, acc[1]);
-    acc[2] = __fmaf_rn(q0.z, b, acc[2]);
-    acc[3] = __fmaf_rn(q0.w, b, acc[3]);
-    acc[4] = __fmaf_rn(q1.x, b, acc[4]);
-    acc[5] = __fmaf_rn(q1.y, b, acc[5]);
-    acc[6] = __fmaf_rn(q1.z, b, acc[6]);
-    acc[7] = __fmaf_rn(q1.w, b, acc[7]);
-    acc[8] = __fmaf_rn(q2.x, b, acc[8]);
-    acc[9] = __fmaf_rn(q2.y, b, acc[9]);
-    acc[10] = __fmaf_rn(q2.z, b, acc[10]);
-    acc[11] = __fmaf_rn(q2.w, b, acc[11]);
-    acc[12] = __fmaf_rn(q3.x, b, acc[12]);
-    acc[13] = __fmaf_rn(q3.y, b, acc[13]);
-    acc[14] = __fmaf_rn(q3.z, b, acc[14]);
-    acc[15] = __fmaf_rn(q3.w, b, acc[15]);
-}
-
-__device__ __forceinline__ void fold16(float (&acc)[16], float (&hi)[16], float (&lo)[16]) {
+// Adds record * b to the lane's sums.  at: offset in the table of the record's chunk
+// lane & 3 (records start at multiples of 64); chunk t ^ (lane & 3) goes to sums
+// 4 t .. 4 t + 3.
+__device__ __forceinline__ void fma_record(const unsigned char *table, uint32_t at, float b,
+                                           uint64_t (&acc)[8]) {
+    const uint64_t bb = pack2(b, b);
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        float s, e;
-        two_sum(hi[i], acc[i], s, e);
-        hi[i] = s;
-        lo[i] = __fadd_rn(lo[i], e);
-        acc[i] = 0.0f;
+    for (uint32_t t = 0; t < 4; t++) {
+        const float4 v = *reinterpret_cast<const float4 *>(table + (at ^ (16u * t)));
+        fma2(acc[2 * t], pack2(v.x, v.y), bb);
+        fma2(acc[2 * t + 1], pack2(v.z, v.w), bb);
+    }
+}
+
+__device__ __forceinline__ void fold_pairs(uint64_t (&acc)[8], float (&hi)[16], float (&lo)[16]) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        float x[2];
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(acc[i]));
+        acc[i] = 0ull;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            float s, e;
+            two_sum(hi[2 * i + c], x[c], s, e);
+            hi[2 * i + c] = s;
+            lo[2 * i + c] = __fadd_rn(lo[2 * i + c], e);
+        }
+    }
+}
+
+// The lane's sums of rows 8 half .. 8 half + 7 (see fma_record) to stage[row of the
+// half * stride + lane].
+__device__ __forceinline__ void stage_sums(const float (&hi)[16], const float (&lo)[16], FF *stage,
+                                           uint32_t stride, uint32_t half) {
+#pragma unroll
+    for (uint32_t t = 0; t < 4; t++) {
+        const uint32_t ch = t ^ (threadIdx.x & 3u);  // rows 4 ch .. 4 ch + 3
+        if (ch >> 1 == half) {
+#pragma unroll
+            for (uint32_t c = 0; c < 4; c++)
+                stage[(4 * (ch & 1u) + c) * stride + threadIdx.x] =
+                    FF{hi[4 * t + c], lo[4 * t + c]};
+        }
     }
 }
 
@@ -139,8 +157,7 @@ __device__ __forceinline__ void combine_lanes(const float (&hi)[16], const float
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; i++) stage[i * THREADS + threadIdx.x] = FF{hi[8 * h + i], lo[8 * h + i]};
+        stage_sums(hi, lo, stage, THREADS, h);
         __syncthreads();
         if (has_col) {
             for (uint32_t i = q; i < 8; i += lpc) {
@@ -152,49 +169,90 @@ __device__ __forceinline__ void combine_lanes(const float (&hi)[16], const float
     }
 }
 
-// Shape of a 16-row work item for a CTA of THREADS threads: THREADS / LPC
-// columns; each warp scatters AP_TI / warps rows, LPR lanes per row, and
-// prefetches NPF entries per lane of each row's next window.  (Scattering rows in
-// 16-byte groups of four entries was measured slower on every workload.)
-template <int THREADS, int LPC>
-struct ApShape {
-    static constexpr int NW = THREADS / 32;
-    static constexpr int TJ = THREADS / LPC;     // column vectors per item
-    static constexpr int RPW = AP_TI / NW;       // rows a warp scatters
-    static constexpr int LPR = 32 / RPW;         // lanes per scattered row
-    static constexpr int NPF = 4;                // prefetched row entries per lane (>= RPW)
-    static_assert(RPW <= NPF, "rows per warp");
-};
+// Named barrier of n threads (0 is __syncthreads).  The aligned form wants each warp
+// converged.
+__device__ __forceinline__ void bar_sync(int id, int n) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+// Parts of segments.  What fixes an item's sums is the partition of its products into
+// FP32 runs: a lane folds its accumulators after every fold / 4 visits of its 4-entry
+// groups, counted from the first window of the segment, where a group that reaches into
+// the next window is visited there again; the runs' sums enter compensated accumulators,
+// in any order.  So a part of a segment's windows can be a CTA's work: it takes the runs
+// whose first visit lies in its windows.  It counts its lanes' visits before them, skips
+// the rest of the run begun there, and goes on past its last window until each of its
+// lanes has finished its own run.  The sums are those of the whole segment, bit for bit up
+// to the order of the compensated additions (sums cut anywhere else differ by 1e-9).  24
+// queries against 160 vectors, 64 segments of which the longest took 68 ms: 14.6 ms.
+//
+// Visits of a lane (the q-th of its column's L, the segment's first group g0) in the
+// windows [s0, w0): one per group that ends by the first entry of w0 (done), and one per
+// window boundary inside a group of the lane.  The column's lanes share the boundaries;
+// cnt: a word of shared memory per lane (the idle ring), l0 the column's first lane.
+constexpr uint32_t AP_STAGE = 2;           // row groups a thread prefetches
+constexpr uint32_t AP_DONE = 0xffffffffu;  // cur of a lane that has no more groups to visit
+
+__device__ __forceinline__ uint32_t visits_before(const uint32_t *__restrict__ cro, uint32_t s0,
+                                                  uint32_t w0, uint32_t g0, uint32_t done,
+                                                  uint32_t l0, uint32_t q, uint32_t L,
+                                                  bool has_col, uint32_t *cnt) {
+    cnt[threadIdx.x] = 0;
+    __syncthreads();
+    if (has_col) {
+        for (uint32_t r = s0 + 1 + q; r <= w0; r += L) {
+            const uint32_t p = __ldg(&cro[r]);
+            if (p & 3u) atomicAdd(&cnt[l0 + ((p >> 2) - g0) % L], 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t n = done + cnt[threadIdx.x];
+    __syncthreads();  // the ring is filled next
+    return n;
+}
 
 // Column side: the item's columns share the lanes evenly (assign_lanes), lpc
 // lanes per column.  Lane q of a column streams the column's 4-entry groups q,
 // q + lpc, q + 2 lpc, ... through its cp.async ring, so the lanes of a column fetch
 // 16 lpc contiguous bytes per load, and keeps its own 16 accumulators for the
 // whole item; the lanes' sums are combined once, at the end of the item.  Row
-// side: lane (srow, sj) of a warp scatters entries sj, sj + LPR, ... of row
-// warp * RPW + srow; the first NPF * LPR entries of each row's next window are
-// prefetched into registers.
-template <int THREADS, int MINB, int LPC>
+// side: a warp group of 128 threads scatters (and clears) its share of the 16 rows, RPG
+// of them side by side in a warp so that a store spreads over 2 RPG banks; a thread takes
+// the 4-entry groups sl, sl + SL, ... of its row, the first AP_STAGE of them prefetched
+// into registers a window ahead (two groups, 256 entries of a row: 6.87 ms for 128 uniform
+// proteomes, 7.05 with one).  A row's entries stay within its warp group, so only
+// the group meets between clearing one window and scattering the next.
+//
+// Bound by the shared-memory pipe at K = 6 (69% of its wavefront rate on 64 uniform
+// proteomes) and by the window barriers where windows are sparse (K = 7: 36%).  128
+// uniform proteomes: 8.21 -> 6.87 ms from the padded records, scalar FMAs and one warp
+// per scattered row this had before.  Not better: masked entries skipped by a branch
+// instead of read from the zero record (7.37), a deeper column ring (6.95), 512- or
+// 1,024-key tables scattered by producer warps while the others gather (9.0, 7.9: every
+// end of a narrower window makes each lane look at a partly used group once more).
+template <int THREADS, int MINB, int LPC, bool PARTS>
 __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
-    using S = ApShape<THREADS, LPC>;
-    constexpr int TJ = S::TJ, RPW = S::RPW, LPR = S::LPR, NPF = S::NPF;
+    constexpr int TJ = THREADS / LPC;            // column vectors per item
+    constexpr uint32_t SL = THREADS / AP_TI;     // threads per row
+    constexpr uint32_t RPG = AP_TI / (THREADS / 128);  // rows per warp group
     constexpr int RING = ring_depth(THREADS);
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t W = 1u << a.wshift, wmask = W - 1u;
-    float *D = reinterpret_cast<float *>(smem);                    // (W + 1) x 16
-    uint4 *ring_k = reinterpret_cast<uint4 *>(smem + (size_t)(W + 1) * D_STRIDE * 4);
+    // the table (W + 1 records) and the column ring
+    float *D = reinterpret_cast<float *>(smem);
+    uint4 *ring_k = reinterpret_cast<uint4 *>(smem + (size_t)(W + 1) * D_REC);
     float4 *ring_v = reinterpret_cast<float4 *>(ring_k + RING * THREADS);
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_lane0[TJ + 1];
     __shared__ uint16_t s_col[THREADS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t srow = lane / LPR, sj = lane % LPR;
-    const uint32_t rr = warp * RPW + srow;  // row position this lane scatters
-    const int rsrc = (int)(srow * LPR);     // first lane of this row
+    const uint32_t wg = threadIdx.x / 128;
+    const uint32_t rr = wg * RPG + threadIdx.x % RPG, sl = threadIdx.x % 128 / RPG;
     const uint32_t Rs = a.R + 1;
+    const uint32_t chunk = 16u * (threadIdx.x & 3u);  // of a record, read first
+    float *drow = D + rr;  // this thread's row of the records
 
-    for (uint32_t i = threadIdx.x; i < (W + 1) * (D_STRIDE / 4); i += THREADS)
-        reinterpret_cast<float4 *>(D)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i = threadIdx.x; i < (W + 1) * (D_REC / 16); i += THREADS)
+        reinterpret_cast<float4 *>(smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     for (;;) {
         __syncthreads();
@@ -202,7 +260,9 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
         __syncthreads();
         const uint32_t it = s_item;
         if (it >= a.nitems) break;
-        const ApItem item = a.items[it];
+        const ApItem item = PARTS ? a.subs[it].item : a.items[it];
+        const uint32_t s0 = PARTS ? a.subs[it].s0 : item.w0;
+        const uint32_t s1 = PARTS ? a.subs[it].s1 : item.w1;
         const int64_t t_start = clock64();
 
         // ---- column side: lpc lanes of column jcol, this one the q-th
@@ -215,103 +275,114 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
         const uint64_t cbase = a.col.vec_off[cv];
         const uint32_t *cro = a.col.roff + (uint64_t)cv * Rs;
         uint32_t c_lo = has_col ? __ldg(&cro[item.w0]) : 0u;
-        const uint32_t c_end = has_col ? __ldg(&cro[item.w1]) : 0u;
+        const uint32_t c_end = has_col ? __ldg(&cro[s1]) : 0u;
         uint32_t c_hi_next = has_col ? __ldg(&cro[item.w0 + 1]) : 0u;
-        // this lane's groups start at entry (c_lo & ~3) + 4q and advance by 16
+        // this lane's groups start at entry (c_s0 & ~3) + 4q of the column, c_s0 its first
+        // entry of the segment, and advance by 4 lpc
         uint32_t cur = (c_lo & ~3u) + 4 * q;  // first entry of the oldest unreleased group
-        uint32_t fetch = cur;                  // next group to fetch
-        uint32_t slot_cur = 0, slot_fetch = 0;
+        int32_t nacc = 0;  // slots added since the last fold; below 0: slots still to skip
+        if (PARTS && item.w0 > s0) {
+            const uint32_t g0 = has_col ? __ldg(&cro[s0]) >> 2 : 0u;
+            const uint32_t ends = (c_lo >> 2) - g0;  // groups of the segment that end by c_lo
+            const uint32_t done = ends > q ? (ends - q + lpc - 1) / lpc : 0u;
+            const uint32_t period = a.fold / 4u;
+            const uint32_t ph =
+                visits_before(cro, s0, item.w0, g0, done, l0, q, lpc, has_col,
+                              reinterpret_cast<uint32_t *>(ring_k)) %
+                period;
+            nacc = ph ? -4 * (int32_t)(period - ph) : 0;
+            cur = 4 * (g0 + q + done * lpc);
+        }
+        uint32_t fetch = cur;  // next group to fetch
+        uint32_t slot_cur = 0;
 #pragma unroll
         for (int k = 0; k < RING; k++) {
             if (fetch < c_end) {
-                cp_async16(&ring_k[slot_fetch * THREADS + threadIdx.x], a.col.keys + cbase + fetch);
-                cp_async16(&ring_v[slot_fetch * THREADS + threadIdx.x], a.col.vals + cbase + fetch);
+                cp_async16(&ring_k[k * THREADS + threadIdx.x], a.col.keys + cbase + fetch);
+                cp_async16(&ring_v[k * THREADS + threadIdx.x], a.col.vals + cbase + fetch);
             }
             fetch += 4 * lpc;
-            slot_fetch = slot_fetch + 1 == RING ? 0 : slot_fetch + 1;
             cp_async_commit();
         }
 
-        // ---- row side: this lane scatters row rr
+        // ---- row side
         const bool has_row = rr < item.nrow;
         const uint32_t rv = has_row ? a.rowids[item.row0 + rr] : 0u;
-        const uint64_t rbase = a.row.vec_off[rv];
+        const uint32_t *rkeys = a.row.keys + a.row.vec_off[rv];
+        const float *rvals = a.row.vals + a.row.vec_off[rv];
         const uint32_t *ro = a.row.roff + (uint64_t)rv * Rs;
-        float acc[16], hi[16], lo[16];
+        uint32_t r_lo = has_row ? __ldg(&ro[item.w0]) : 0u;       // row entries of window r
+        uint32_t r_hi = has_row ? __ldg(&ro[item.w0 + 1]) : 0u;
+        uint32_t r_hi_next = has_row ? __ldg(&ro[min(item.w0 + 2, a.R)]) : 0u;
+        // this thread's first groups of row entries [lo, hi)
+        uint4 pk[AP_STAGE];
+        float4 pv[AP_STAGE];
+        auto prefetch_row = [&](uint32_t lo, uint32_t hi) {
 #pragma unroll
-        for (int i = 0; i < 16; i++) acc[i] = hi[i] = lo[i] = 0.0f;
-        uint32_t nacc = 0;
+            for (uint32_t k = 0; k < AP_STAGE; k++) {
+                const uint32_t e = 4u * ((lo >> 2) + sl + k * SL);
+                if (e < hi) {
+                    pk[k] = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
+                    pv[k] = __ldg(reinterpret_cast<const float4 *>(rvals + e));
+                }
+            }
+        };
+        prefetch_row(r_lo, r_hi);
+        uint64_t acc[8];
+        float hi[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = 0ull;
+#pragma unroll
+        for (int i = 0; i < 16; i++) hi[i] = lo[i] = 0.0f;
 
-        // window offsets of LPR windows, held by the row's lanes; the first
-        // NPF * LPR entries of the row's next window prefetched, NPF per lane
-        uint32_t wb = item.w0;
-        uint32_t r_lo = 0, r_hi = 0;
-        if (has_row) {
-            r_lo = __ldg(&ro[min(wb + sj, a.R)]);
-            r_hi = __ldg(&ro[min(wb + sj + 1, a.R)]);
-        }
-        uint32_t pk[NPF];
-        float pv[NPF];
-        {
-            const uint32_t lo0 = __shfl_sync(0xffffffffu, r_lo, rsrc);
-            const uint32_t hi0 = __shfl_sync(0xffffffffu, r_hi, rsrc);
+        for (uint32_t r = item.w0; r < s1; r++) {
+            // scatter window r of row rr: prefetched groups, the rest loaded.  held: window
+            // offsets of the prefetched entries, to clear them (W: none)
+            uint32_t held[2 * AP_STAGE];
 #pragma unroll
-            for (int t = 0; t < NPF; t++) {
-                const uint32_t e = lo0 + sj + t * LPR;
-                pk[t] = 0xffffffffu;
-                pv[t] = 0.f;
-                if (has_row && e < hi0) {
-                    pk[t] = __ldg(&a.row.keys[rbase + e]);
-                    pv[t] = __ldg(&a.row.vals[rbase + e]);
-                }
-            }
-        }
-
-        for (uint32_t r = item.w0; r < item.w1; r++) {
-            const int sl = (int)(r - wb);
-            const uint32_t lo_r = __shfl_sync(0xffffffffu, r_lo, rsrc + sl);
-            const uint32_t hi_r = __shfl_sync(0xffffffffu, r_hi, rsrc + sl);
-            // scatter window r of row rr: first NPF * LPR entries from registers, the rest loaded
-            uint32_t ck[NPF];
+            for (uint32_t k = 0; k < AP_STAGE; k++) {
+                const uint32_t e = 4u * ((r_lo >> 2) + sl + k * SL);
+                held[2 * k] = held[2 * k + 1] = W | W << 16;
+                if (e < r_hi) {
+                    const uint32_t ks[4] = {pk[k].x, pk[k].y, pk[k].z, pk[k].w};
+                    const float vs[4] = {pv[k].x, pv[k].y, pv[k].z, pv[k].w};
+                    uint32_t off[4];
 #pragma unroll
-            for (int t = 0; t < NPF; t++) {
-                ck[t] = pk[t];
-                if (pk[t] != 0xffffffffu) D[d_slot(pk[t] & wmask, rr)] = pv[t];
-            }
-            if (has_row) {
-                for (uint32_t e = lo_r + NPF * LPR + sj; e < hi_r; e += LPR) {
-                    const uint32_t key = __ldg(&a.row.keys[rbase + e]);
-                    D[d_slot(key & wmask, rr)] = __ldg(&a.row.vals[rbase + e]);
-                }
-            }
-            // prefetch the next window's row offsets and first entries
-            if (r + 1 < item.w1) {
-                if (r + 1 - wb >= (uint32_t)LPR) {
-                    wb = r + 1;
-                    if (has_row) {
-                        r_lo = __ldg(&ro[min(wb + sj, a.R)]);
-                        r_hi = __ldg(&ro[min(wb + sj + 1, a.R)]);
+                    for (uint32_t u = 0; u < 4; u++) {
+                        const bool in = e + u >= r_lo && e + u < r_hi;
+                        off[u] = in ? ks[u] & wmask : W;
+                        if (in) drow[off[u] * AP_TI] = vs[u];
                     }
+                    held[2 * k] = off[0] | off[1] << 16;
+                    held[2 * k + 1] = off[2] | off[3] << 16;
                 }
-                const int sn = (int)(r + 1 - wb);
-                const uint32_t nlo = __shfl_sync(0xffffffffu, r_lo, rsrc + sn);
-                const uint32_t nhi = __shfl_sync(0xffffffffu, r_hi, rsrc + sn);
+            }
+            const uint32_t rest = 4u * ((r_lo >> 2) + sl + AP_STAGE * SL);
+            const uint32_t rest_hi = r_hi;
+            for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
+                const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
+                const float4 vv = __ldg(reinterpret_cast<const float4 *>(rvals + e));
+                const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
+                const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
 #pragma unroll
-                for (int t = 0; t < NPF; t++) {
-                    const uint32_t e = nlo + sj + t * LPR;
-                    pk[t] = 0xffffffffu;
-                    if (has_row && e < nhi) {
-                        pk[t] = __ldg(&a.row.keys[rbase + e]);
-                        pv[t] = __ldg(&a.row.vals[rbase + e]);
-                    }
-                }
-                // the rest of the row's next window (the scatter loop's loads) into L2,
-                // a whole window's gathers ahead: large rows stream from DRAM
-                if (has_row && sj == 0 && nhi > nlo + NPF * LPR)
-                    prefetch_l2(a.row.keys + rbase, a.row.vals + rbase, nlo + NPF * LPR, nhi);
+                for (uint32_t u = 0; u < 4; u++)
+                    if (e + u < rest_hi) drow[(ks[u] & wmask) * AP_TI] = vs[u];
+            }
+            // the next window's row entries
+            r_lo = r_hi;
+            r_hi = r_hi_next;
+            if (r + 1 < s1) {
+                prefetch_row(r_lo, r_hi);
+                // the rest of it (the loop's loads) into L2, a whole window's gathers ahead:
+                // large rows stream from DRAM
+                if (sl == 0 && (r_lo & ~3u) + 4u * AP_STAGE * SL < r_hi)
+                    prefetch_l2(rkeys, rvals, (r_lo & ~3u) + 4u * AP_STAGE * SL, r_hi);
+                if (has_row && r + 3 <= a.R) r_hi_next = __ldg(&ro[r + 3]);
             }
             const uint32_t c_hi = c_hi_next;
             if (has_col && r + 2 <= a.R) c_hi_next = __ldg(&cro[r + 2]);
+            // past the part's own windows only the lanes inside a run go on
+            if (PARTS && r >= item.w1 && nacc <= 0) cur = AP_DONE;
             __syncthreads();
             // this lane's groups of the column that start before c_hi
             if (has_col) {
@@ -321,47 +392,60 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
                     const float4 vv = ring_v[slot_cur * THREADS + threadIdx.x];
                     const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
                     const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
+                    const uint32_t first = PARTS && nacc < 0 ? AP_DONE : c_lo;  // skipped: adds nothing
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         const uint32_t e = cur + u;
-                        const bool ok = e >= c_lo && e < c_hi;
-                        fma_entry(D, ok ? (ks[u] & wmask) : W, ok ? vs[u] : 0.0f, acc);
+                        const bool ok = e >= first && e < c_hi;
+                        fma_record(smem, chunk + (ok ? ks[u] & wmask : W) * D_REC,
+                                   ok ? vs[u] : 0.0f, acc);
                     }
                     nacc += 4;
-                    if (nacc >= a.fold) {
-                        fold16(acc, hi, lo);
+                    if (nacc >= (int32_t)a.fold) {
+                        fold_pairs(acc, hi, lo);
                         nacc = 0;
+                        if (PARTS && r >= item.w1) {
+                            cur = AP_DONE;
+                            break;
+                        }
                     }
                     if (cur + 4 > c_hi) break;  // reaches into the next window: keep it
                     if (fetch < c_end) {
-                        cp_async16(&ring_k[slot_fetch * THREADS + threadIdx.x],
+                        cp_async16(&ring_k[slot_cur * THREADS + threadIdx.x],
                                    a.col.keys + cbase + fetch);
-                        cp_async16(&ring_v[slot_fetch * THREADS + threadIdx.x],
+                        cp_async16(&ring_v[slot_cur * THREADS + threadIdx.x],
                                    a.col.vals + cbase + fetch);
                     }
                     fetch += 4 * lpc;
-                    slot_fetch = slot_fetch + 1 == RING ? 0 : slot_fetch + 1;
                     cp_async_commit();
                     cur += 4 * lpc;
                     slot_cur = slot_cur + 1 == RING ? 0 : slot_cur + 1;
                 }
             }
             c_lo = c_hi;
-            __syncthreads();
+            bool more = true;
+            if (!PARTS || r + 1 < item.w1)
+                __syncthreads();
+            else  // a lane inside a run with entries of the segment left
+                more = __syncthreads_or(nacc > 0 && cur != AP_DONE && c_lo < c_end);
             // clear window r of row rr
 #pragma unroll
-            for (int t = 0; t < NPF; t++)
-                if (ck[t] != 0xffffffffu) D[d_slot(ck[t] & wmask, rr)] = 0.0f;
-            if (has_row) {
-                for (uint32_t e = lo_r + NPF * LPR + sj; e < hi_r; e += LPR) {
-                    const uint32_t key = __ldg(&a.row.keys[rbase + e]);
-                    D[d_slot(key & wmask, rr)] = 0.0f;
-                }
+            for (uint32_t k = 0; k < 2 * AP_STAGE; k++) {
+                if ((held[k] & 0xffffu) != W) drow[(held[k] & 0xffffu) * AP_TI] = 0.0f;
+                if (held[k] >> 16 != W) drow[(held[k] >> 16) * AP_TI] = 0.0f;
             }
-            __syncwarp();
+            for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
+                const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
+                const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++)
+                    if (e + u < rest_hi) drow[(ks[u] & wmask) * AP_TI] = 0.0f;
+            }
+            if (PARTS && !more) break;
+            bar_sync(1 + (int)wg, 128);
         }
         cp_async_wait_all();
-        fold16(acc, hi, lo);
+        fold_pairs(acc, hi, lo);
         combine_lanes<THREADS>(hi, lo, reinterpret_cast<FF *>(ring_k),
                                a.part + (uint64_t)item.part * (AP_TI * TJ), TJ, has_col, jcol, l0,
                                q, lpc);
@@ -631,7 +715,8 @@ static int ap_lpc(int tile_cols) { return tile_cols == 256 ? 2 : AP_LPC; }
 
 size_t ap_smem_bytes(uint32_t wshift, int tile_rows, int tile_cols) {
     if (tile_rows == 32) return r32_smem_bytes(wshift);
-    return (((size_t)1 << wshift) + 1) * D_STRIDE * sizeof(float) +
+    // (the 64- and 32-column shapes' callers were told 80 bytes per record)
+    return (((size_t)1 << wshift) + 1) * (tile_cols >= 128 ? D_REC : 80u) +
            ap_ring_bytes(tile_cols * ap_lpc(tile_cols));
 }
 
@@ -645,19 +730,27 @@ int ap_threads(uint32_t wshift, int tile_rows, int tile_cols) {
     return tile_cols * ap_lpc(tile_cols);
 }
 
-static const void *ap_kernel(uint32_t wshift, int tile_rows, int tile_cols) {
+static const void *ap_kernel(uint32_t wshift, int tile_rows, int tile_cols, bool parts) {
     if (tile_rows == 32)
         return r32_wide(wshift) ? (const void *)k_allpairs32<512, 1>
                                 : (const void *)k_allpairs32<256, 2>;
-    if (tile_cols == 256) return (const void *)k_allpairs<512, 1, 2>;
-    if (tile_cols == 128) return (const void *)k_allpairs<512, 1, 4>;
-    return tile_cols == 32 ? (const void *)k_allpairs<128, 4, 4> : (const void *)k_allpairs<256, 2, 4>;
+    if (tile_cols == 256)
+        return parts ? (const void *)k_allpairs<512, 1, 2, true>
+                     : (const void *)k_allpairs<512, 1, 2, false>;
+    if (tile_cols == 128)
+        return parts ? (const void *)k_allpairs<512, 1, 4, true>
+                     : (const void *)k_allpairs<512, 1, 4, false>;
+    return tile_cols == 32 ? (const void *)k_allpairs<128, 4, 4, false>
+                           : (const void *)k_allpairs<256, 2, 4, false>;
 }
 
 cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_per_sm) {
     const size_t smem = ap_smem_bytes(wshift, tile_rows, tile_cols);
-    const void *fn = ap_kernel(wshift, tile_rows, tile_cols);
+    const void *fn = ap_kernel(wshift, tile_rows, tile_cols, false);
     PHYLO_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (tile_rows == AP_TI && tile_cols >= 128)
+        PHYLO_CHECK(cudaFuncSetAttribute(ap_kernel(wshift, tile_rows, tile_cols, true),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (ctas_per_sm) {
         int n = 0;
         PHYLO_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -668,22 +761,11 @@ cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_
 }
 
 cudaError_t ap_launch(const ApArgs &a, int tile_rows, int tile_cols, int grid, cudaStream_t st) {
-    const size_t smem = ap_smem_bytes(a.wshift, tile_rows, tile_cols);
-    if (tile_rows == 32) {
-        if (r32_wide(a.wshift))
-            k_allpairs32<512, 1><<<grid, 512, smem, st>>>(a);
-        else
-            k_allpairs32<256, 2><<<grid, 256, smem, st>>>(a);
-    } else if (tile_cols == 256) {
-        k_allpairs<512, 1, 2><<<grid, 512, smem, st>>>(a);
-    } else if (tile_cols == 128) {
-        k_allpairs<512, 1, 4><<<grid, 512, smem, st>>>(a);
-    } else if (tile_cols == 32) {
-        k_allpairs<128, 4, 4><<<grid, 128, smem, st>>>(a);
-    } else {
-        k_allpairs<256, 2, 4><<<grid, 256, smem, st>>>(a);
-    }
-    return cudaGetLastError();
+    ApArgs arg = a;
+    void *argv[] = {&arg};
+    return cudaLaunchKernel(ap_kernel(a.wshift, tile_rows, tile_cols, a.subs != nullptr),
+                            dim3(grid), dim3(ap_threads(a.wshift, tile_rows, tile_cols)), argv,
+                            ap_smem_bytes(a.wshift, tile_rows, tile_cols), st);
 }
 
 // ---------------------------------------------------------------------------
@@ -759,24 +841,42 @@ cudaError_t range_index_launch(const uint32_t *keys, const uint64_t *vec_off, ui
 // reduction of partial blocks
 // ---------------------------------------------------------------------------
 
-// grid = (ntiles, tile rows), block = tile columns: one (row, column) pair per
-// thread, its S partials summed in segment order (double-double), so the result
-// does not depend on how the items were scheduled.
-__global__ void k_ap_reduce(ApReduceArgs r) {
-    const ApTile t = r.tiles[blockIdx.x];
-    const uint32_t c = threadIdx.x, i = blockIdx.y;
-    if (c >= t.ncol || i >= t.nrow) return;
-    const uint32_t rowpos = t.row0 + i, colpos = t.col0 + c;
-    if (r.upper == 1 && !(rowpos < colpos)) return;
-    if (r.upper == 2 && !(rowpos <= colpos)) return;  // with the diagonal
-    const uint64_t blk = (uint64_t)r.ti * r.tj;  // float pairs per partial block
-    const FF *base = r.part + (uint64_t)blockIdx.x * r.S * blk + i * r.tj + c;
+// grid = (ntiles, tile rows), block = (tile columns, AP_RED): one (row, column) pair per
+// threadIdx.x, its partials split evenly over threadIdx.y; each share is summed in
+// part order and the shares in order (double-double), so the result does not depend on
+// how the items were scheduled.  Bound by the latency of a pair's chain of partials, so
+// the chain is cut in AP_RED (one thread per pair: 107 us for 8 tiles of 152 partial
+// blocks, 128 uniform proteomes).
+constexpr int AP_RED = 4;
+__global__ void __launch_bounds__(256 * AP_RED) k_ap_reduce(ApReduceArgs r) {
+    __shared__ DD s_acc[AP_RED - 1][256];
+    const uint32_t *t = r.tiles + (uint64_t)blockIdx.x * r.tile_words;
+    const uint32_t row0 = t[0], nrow = t[1], col0 = t[2], ncol = t[3];
+    const uint64_t part0 = r.tile_words == 8 ? t[4] : (uint64_t)blockIdx.x * r.S;
+    const uint32_t S = r.tile_words == 8 ? t[5] : r.S;
+    const uint32_t c = threadIdx.x, i = blockIdx.y, y = threadIdx.y;
+    const uint32_t rowpos = row0 + i, colpos = col0 + c;
+    bool use = c < ncol && i < nrow;
+    if (r.upper == 1 && !(rowpos < colpos)) use = false;
+    if (r.upper == 2 && !(rowpos <= colpos)) use = false;  // with the diagonal
     DD acc = {0.0, 0.0};
-    for (uint32_t s = 0; s < r.S; s++) {
-        const FF p = base[(uint64_t)s * blk];
-        dd_add(acc, (double)p.hi);
-        dd_add(acc, (double)p.lo);
+    if (use) {
+        const uint64_t blk = (uint64_t)r.ti * r.tj;  // float pairs per partial block
+        const FF *base = r.part + part0 * blk + i * r.tj + c;
+        const uint32_t b0 = (uint32_t)((uint64_t)y * S / AP_RED);
+        const uint32_t b1 = (uint32_t)((uint64_t)(y + 1) * S / AP_RED);
+#pragma unroll 8
+        for (uint32_t s = b0; s < b1; s++) {
+            const FF p = base[(uint64_t)s * blk];
+            dd_add(acc, (double)p.hi);
+            dd_add(acc, (double)p.lo);
+        }
+        if (y) s_acc[y - 1][c] = acc;
     }
+    __syncthreads();
+    if (!use || y) return;
+#pragma unroll
+    for (int k = 0; k < AP_RED - 1; k++) acc = dd_merge(acc, s_acc[k][c]);
     const double v = __dadd_rn(acc.hi, acc.lo);
     const uint32_t rowid = r.rowids[rowpos], colid = r.colids[colpos];
     r.out[(uint64_t)rowid * r.ldc + colid] = v;
@@ -785,7 +885,7 @@ __global__ void k_ap_reduce(ApReduceArgs r) {
 
 cudaError_t ap_reduce_launch(const ApReduceArgs &r, cudaStream_t st) {
     if (r.ntiles == 0) return cudaSuccess;
-    k_ap_reduce<<<dim3(r.ntiles, r.ti), r.tj, 0, st>>>(r);
+    k_ap_reduce<<<dim3(r.ntiles, r.ti), dim3(r.tj, AP_RED), 0, st>>>(r);
     return cudaGetLastError();
 }
 

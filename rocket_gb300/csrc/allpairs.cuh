@@ -17,6 +17,13 @@ struct ApItem {
     uint32_t tile;        // tile this item contributes to
 };
 
+// A part [item.w0, item.w1) of the segment [s0, s1) of a tile's windows, computed by a
+// CTA of its own with the sums the whole segment would form (k_allpairs).
+struct ApSubItem {
+    ApItem item;
+    uint32_t s0, s1, unused0, unused1;
+};
+
 // Rows and columns may live in different arenas (e.g. arriving queries against
 // a resident database); for all pairs of one arena both sides are the same.
 struct ApArena {
@@ -31,7 +38,8 @@ struct ApArgs {
     uint32_t R;                // windows per vector
     uint32_t wshift;           // window width = 1 << wshift keys
     const uint32_t *rowids, *colids;
-    const ApItem *items;
+    const ApItem *items;       // whole segments, or (null)
+    const ApSubItem *subs;     // parts of segments (16 x 128 and 16 x 256 tiles)
     uint32_t nitems;
     uint32_t *counter;         // work counter (zeroed before launch)
     FF *part;                  // [parts][tile rows][tile cols]
@@ -40,7 +48,7 @@ struct ApArgs {
 };
 
 // Tile shapes (tile_rows x tile_cols) select the kernel: 16 x 128 (512 threads),
-// 16 x 64 (256) and 16 x 32 (128) use 80-byte key records and four lanes per column,
+// 16 x 64 (256) and 16 x 32 (128) use 64-byte key records and four lanes per column,
 // 16 x 256 (512 threads) the same records and two lanes per column; 32 x 64 uses
 // 128-byte swizzled records and eight lanes per column.
 bool ap_shape_ok(int tile_rows, int tile_cols);
@@ -56,7 +64,8 @@ cudaError_t range_index_launch(const uint32_t *keys, const uint64_t *vec_off, ui
                                uint64_t max_len);
 
 // Tile t (rows rowids[row0..], columns colids[col0..]) has S partial blocks
-// part[t * S + s].  Writes out[rowid * ldc + colid] (and the mirrored entry
+// part[t * S + s] (tiles of 4 words), or nparts of its own from part0 (tiles of 8
+// words: ApTile, part0, nparts, two unused).  Writes out[rowid * ldc + colid] (and the mirrored entry
 // when `mirror`), for pairs with row position < column position when `upper` is
 // 1, <= when it is 2.
 struct ApTile {
@@ -64,8 +73,8 @@ struct ApTile {
 };
 struct ApReduceArgs {
     const FF *part;            // blocks of ti x tj float pairs
-    const ApTile *tiles;
-    uint32_t ntiles, S, ti, tj;
+    const uint32_t *tiles;     // ntiles x tile_words
+    uint32_t ntiles, tile_words, S, ti, tj;
     const uint32_t *rowids, *colids;
     double *out;
     uint64_t ldc;

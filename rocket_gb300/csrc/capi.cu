@@ -489,15 +489,16 @@ int phyloPairsThreads(int window_shift, int tile_rows, int tile_cols) {
 // row vectors come from the row arena, column vectors from the column arena
 // (the same arena for all pairs of one set).  d_counter must be zero.
 // d_item_cycles may be 0.
-int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
-                     uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
-                     uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,
-                     unsigned int num_windows, int window_shift, uintptr_t d_rowids,
-                     uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
-                     uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
-                     int tile_cols, int grid) {
+static int pairs_launch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
+                        uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
+                        uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,
+                        unsigned int num_windows, int window_shift, uintptr_t d_rowids,
+                        uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
+                        uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
+                        int tile_cols, int grid, bool parts) {
     if (!ap_shape_ok(tile_rows, tile_cols) || window_shift < 4 ||
-        window_shift > ap_max_wshift(tile_rows, tile_cols) || num_items < 0 || grid <= 0)
+        window_shift > ap_max_wshift(tile_rows, tile_cols) || num_items < 0 || grid <= 0 ||
+        (parts && (tile_rows != AP_TI || tile_cols < 128)))
         return (int)cudaErrorInvalidValue;
     ApArgs a;
     a.row.keys = (const uint32_t *)d_row_keys;
@@ -512,7 +513,8 @@ int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_val
     a.wshift = (uint32_t)window_shift;
     a.rowids = (const uint32_t *)d_rowids;
     a.colids = (const uint32_t *)d_colids;
-    a.items = (const ApItem *)d_items;
+    a.items = parts ? nullptr : (const ApItem *)d_items;
+    a.subs = parts ? (const ApSubItem *)d_items : nullptr;
     a.nitems = (uint32_t)num_items;
     a.counter = (uint32_t *)d_counter;
     a.part = (FF *)d_part;
@@ -522,17 +524,45 @@ int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_val
     return (int)ap_launch(a, tile_rows, tile_cols, grid, (cudaStream_t)stream);
 }
 
-// Sums the partial blocks of each tile (4 uint32 per tile: row0, nrow, col0, ncol).
-int phyloPairsReduce(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
-                     int segments, int tile_rows, int tile_cols, uintptr_t d_rowids,
-                     uintptr_t d_colids, uintptr_t d_out, long ldc, int upper, int mirror) {
+int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
+                     uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
+                     uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,
+                     unsigned int num_windows, int window_shift, uintptr_t d_rowids,
+                     uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
+                     uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
+                     int tile_cols, int grid) {
+    return pairs_launch(stream, d_row_keys, d_row_values, d_row_vec_off, d_row_roff, d_col_keys,
+                        d_col_values, d_col_vec_off, d_col_roff, num_windows, window_shift,
+                        d_rowids, d_colids, d_items, num_items, d_counter, d_part, fold,
+                        d_item_cycles, tile_rows, tile_cols, grid, false);
+}
+
+// The same over parts of segments (12 uint32 each, see ApSubItem).
+int phyloPairsLaunchParts(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
+                          uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
+                          uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,
+                          unsigned int num_windows, int window_shift, uintptr_t d_rowids,
+                          uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
+                          uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
+                          int tile_cols, int grid) {
+    return pairs_launch(stream, d_row_keys, d_row_values, d_row_vec_off, d_row_roff, d_col_keys,
+                        d_col_values, d_col_vec_off, d_col_roff, num_windows, window_shift,
+                        d_rowids, d_colids, d_items, num_items, d_counter, d_part, fold,
+                        d_item_cycles, tile_rows, tile_cols, grid, true);
+}
+
+static int pairs_reduce(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
+                        int tile_words, int segments, int tile_rows, int tile_cols,
+                        uintptr_t d_rowids, uintptr_t d_colids, uintptr_t d_out, long ldc,
+                        int upper, int mirror) {
     if (!ap_shape_ok(tile_rows, tile_cols) || upper < 0 || upper > 2 || num_tiles < 0 ||
         (num_tiles > 0 && segments <= 0) || ldc <= 0)
         return (int)cudaErrorInvalidValue;
     ApReduceArgs r;
     r.part = (const FF *)d_part;
-    r.tiles = (const ApTile *)d_tiles;
+    r.tiles = (const uint32_t *)d_tiles;
     r.ntiles = (uint32_t)num_tiles;
+    r.tile_words = (uint32_t)tile_words;
     r.S = (uint32_t)segments;
     r.ti = (uint32_t)tile_rows;
     r.tj = (uint32_t)tile_cols;
@@ -543,6 +573,23 @@ int phyloPairsReduce(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int 
     r.upper = upper;
     r.mirror = mirror;
     return (int)ap_reduce_launch(r, (cudaStream_t)stream);
+}
+
+// Sums the partial blocks of each tile (4 uint32 per tile: row0, nrow, col0, ncol).
+int phyloPairsReduce(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
+                     int segments, int tile_rows, int tile_cols, uintptr_t d_rowids,
+                     uintptr_t d_colids, uintptr_t d_out, long ldc, int upper, int mirror) {
+    return pairs_reduce(stream, d_part, d_tiles, num_tiles, 4, segments, tile_rows, tile_cols,
+                        d_rowids, d_colids, d_out, ldc, upper, mirror);
+}
+
+// The same for tiles with their own partial blocks (8 uint32 per tile: row0, nrow, col0,
+// ncol, part0, nparts, two unused).
+int phyloPairsReduceParts(uintptr_t stream, uintptr_t d_part, uintptr_t d_tiles, int num_tiles,
+                          int tile_rows, int tile_cols, uintptr_t d_rowids, uintptr_t d_colids,
+                          uintptr_t d_out, long ldc, int upper, int mirror) {
+    return pairs_reduce(stream, d_part, d_tiles, num_tiles, 8, 1, tile_rows, tile_cols, d_rowids,
+                        d_colids, d_out, ldc, upper, mirror);
 }
 
 // ---------------------------------------------------------------------------

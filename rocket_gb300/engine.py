@@ -35,6 +35,10 @@ from ._native import check
 
 AP_TI = 16          # default rows per work item (16 or 32: selects the pair kernel)
 AP_TJ = 128         # default column vectors per work item (512-thread CTAs)
+PART_WINDOWS = 128  # windows per part of a segment fixed by EngineConfig.segments, at most
+                    # (24 queries x 160 vectors in 16 segments: 14.6 ms; 15.2 / 15.8 / 18.9
+                    # with 64 / 256 / 512)
+PART_SETUP = 2.0    # cost of starting and ending an item, in windows
 NSYM = {"protein": 21, "DNA": 4}
 
 
@@ -58,6 +62,27 @@ def auto_tile_cols(n_cols: int) -> int:
     full; in a triangle over fewer than 384 vectors most 256-column items would be
     half empty, and 128-column items keep more lanes busy."""
     return 256 if n_cols >= 384 else 128
+
+
+def split_segments(windows: np.ndarray, est: np.ndarray, tail: np.ndarray, grid: int,
+                   most: int) -> np.ndarray:
+    """Parts per segment of a window plan with too few segments to fill the GPU.  A part
+    is computed by a CTA of its own with the sums the whole segment would form
+    (phyloPairsLaunchParts).  ``windows``: windows of each segment; ``est``: its cost;
+    ``tail``: windows a part goes on past its own to finish its lanes' FP32 runs.  Of
+    several totals up to ``most`` items, the one whose items, PART_SETUP windows and a
+    tail longer than their share, finish first on ``grid`` CTAs, longest first."""
+    best, best_time = None, math.inf
+    total = est.sum()
+    for goal in (0, 1, 2, 4, most / grid):
+        n = np.ceil(est * (goal * grid / total)) if goal else np.ones(len(est))
+        n = np.clip(n, 1, windows).astype(np.int64)
+        extra = np.where(n > 1, PART_SETUP + tail, PART_SETUP)
+        cost = np.sort(np.repeat(est * (1.0 / n + extra / windows), n))[::-1]
+        time = cost[::grid].sum()
+        if time < best_time:
+            best, best_time = n, time
+    return best
 
 
 # --------------------------------------------------------------------------
@@ -379,6 +404,10 @@ class PairPlan:
     host_tiles: np.ndarray = field(default=None)
     item_tile: np.ndarray = field(default=None)  # tile of each item (launch order)
     item_share: np.ndarray = field(default=None)  # fraction of its tile's windows per item
+    host_parts: np.ndarray = field(default=None)  # int64 [n, 12]: the items cut into parts, or None
+    host_part_tiles: np.ndarray = field(default=None)  # int64 [ntiles, 8] with parts
+    parts: torch.Tensor = None       # int32 device copies of both
+    part_tiles: torch.Tensor = None
 
 
 @dataclass
@@ -644,7 +673,13 @@ class PairEngine:
         item_tile = t_of[order]
         share = share[order]
         dev = self.device
-        return PairPlan(
+        cut = None
+        if self.cfg.algorithm == "window" and self.cfg.tile_rows == AP_TI and \
+                self.cfg.tile_cols >= 128:
+            cut = self._cut_items(items, est, host_tiles, col_nnz[colids])
+            if cut is not None:
+                nparts = len(cut[0])
+        plan = PairPlan(
             rowids=torch.from_numpy(rowids.astype(np.int32)).to(dev),
             colids=torch.from_numpy(colids.astype(np.int32)).to(dev),
             tiles=torch.from_numpy(host_tiles.astype(np.int32)).to(dev),
@@ -653,6 +688,50 @@ class PairEngine:
             est=est, pairs=pairs, host_items=items, algorithm=self.cfg.algorithm,
             nparts=nparts, host_rowids=rowids, host_colids=colids, host_tiles=host_tiles,
             item_tile=item_tile, item_share=share)
+        if cut is not None:
+            plan.host_parts, plan.host_part_tiles = cut
+            plan.parts = torch.from_numpy(plan.host_parts.astype(np.int32)).to(dev)
+            plan.part_tiles = torch.from_numpy(plan.host_part_tiles.astype(np.int32)).to(dev)
+        return plan
+
+    def _cut_items(self, items, est, host_tiles, nnz_of_col):
+        """(parts [n, 12], tiles [ntiles, 8]) of a plan whose items are too few to fill the
+        GPU, longest first, or None where no item is cut.  ``items`` in launch order;
+        ``nnz_of_col``: entries of the plan's columns in their order, most first."""
+        goal = self.cfg.items_per_cta * self.grid
+        fixed = self.cfg.segments > 0
+        if len(items) == 0 or (not fixed and len(items) >= goal):
+            return None
+        windows = items[:, 5] - items[:, 4]
+        # a part goes on past its own windows until each of its lanes has finished the FP32
+        # run it is in: the windows in which the tile's sparsest column has one per lane
+        least = nnz_of_col[items[:, 2] + items[:, 3] - 1] / max(self.arena.R, 1)
+        tail = self.cfg.fold * -(-512 // np.maximum(items[:, 3], 1)) / np.maximum(least, 1e-9)
+        if fixed:  # as the columns ask, so a pair's arithmetic does not depend on the rows
+            n = np.minimum(-(-windows // PART_WINDOWS), windows / np.maximum(4.0 * tail, 1.0))
+            n = np.maximum(n, 1).astype(np.int64)
+        else:
+            n = split_segments(windows, est, tail, self.grid, goal)
+        if n.max() == 1:
+            return None
+        order = np.argsort(items[:, 6], kind="stable")  # tiles in order, segments in order
+        first = np.empty(len(items), np.int64)
+        first[order] = np.cumsum(n[order]) - n[order]
+        of = np.repeat(np.arange(len(items)), n)        # item of each part, and its number
+        k = np.arange(len(of)) - np.repeat(np.cumsum(n) - n, n)
+        parts = np.zeros((len(of), 12), np.int64)
+        parts[:, 0:4] = items[of, 0:4]
+        parts[:, 4] = items[of, 4] + k * windows[of] // n[of]
+        parts[:, 5] = items[of, 4] + (k + 1) * windows[of] // n[of]
+        parts[:, 6] = first[of] + k
+        parts[:, 7] = items[of, 7]
+        parts[:, 8] = items[of, 4]
+        parts[:, 9] = items[of, 5]
+        tiles = np.zeros((len(host_tiles), 8), np.int64)
+        tiles[:, 0:4] = host_tiles[:, 0:4]
+        tiles[:, 5] = np.bincount(items[:, 7], weights=n, minlength=len(host_tiles))
+        tiles[:, 4] = np.cumsum(tiles[:, 5]) - tiles[:, 5]
+        return parts[np.argsort(-(est / n)[of], kind="stable")], tiles
 
     def plan_triangle(self, ids: Optional[Sequence[int]] = None, ldc: Optional[int] = None) -> PairPlan:
         """All pairs i < j among ``ids`` (default: every vector of the arena), and
@@ -686,7 +765,7 @@ class PairEngine:
         if plan.algorithm == "postings":
             need = plan.nparts * self.cfg.block * self.cfg.block * 2  # int64 as int32 pairs
         else:
-            need = plan.ntiles * plan.S * self.cfg.tile_rows * self.cfg.tile_cols * 2
+            need = max(plan.nparts, plan.ntiles * plan.S) * self.cfg.tile_rows * self.cfg.tile_cols * 2
         if self.part is None or self.part.numel() < need:
             self.part = torch.empty(max(need, 2), dtype=torch.float32, device=self.device)
         return self.part
@@ -711,6 +790,7 @@ class PairEngine:
             raise ValueError("dense key ranks need rows and columns in the same arena "
                              "(EngineConfig(compress=False) for two arenas)")
         cyc = _p(item_cycles) if item_cycles is not None else 0
+        parts = plan.host_parts is not None and item_cycles is None  # cycles are per whole item
         if plan.algorithm == "postings":
             check(self.L.phyloPostingsLaunch(
                 st, _p(a.pair_keys()), _p(a.values), _p(a.vec_off), _p(a.roff),
@@ -724,18 +804,27 @@ class PairEngine:
                 _p(plan.colids), _p(out), plan.ldc, int(plan.diag and diagonal),
                 int(plan.mirror)))
         else:
-            check(self.L.phyloPairsLaunch(
+            launch = self.L.phyloPairsLaunchParts if parts else self.L.phyloPairsLaunch
+            check(launch(
                 st, _p(a.pair_keys()), _p(a.values), _p(a.vec_off), _p(a.roff),
                 _p(ca.pair_keys()), _p(ca.values), _p(ca.vec_off), _p(ca.roff), a.R,
-                self.cfg.wshift, _p(plan.rowids), _p(plan.colids), _p(plan.items), plan.nitems,
+                self.cfg.wshift, _p(plan.rowids), _p(plan.colids),
+                _p(plan.parts if parts else plan.items), plan.nparts if parts else plan.nitems,
                 _p(self.counter), _p(part), self.cfg.fold, cyc, self.cfg.tile_rows,
                 self.cfg.tile_cols, self.grid))
             if events is not None:
                 events[1].record(s_obj)
-            check(self.L.phyloPairsReduce(
-                st, _p(part), _p(plan.tiles), plan.ntiles, plan.S, self.cfg.tile_rows,
-                self.cfg.tile_cols, _p(plan.rowids), _p(plan.colids), _p(out), plan.ldc,
-                (2 if plan.diag and diagonal else 1) if plan.upper else 0, int(plan.mirror)))
+            upper = (2 if plan.diag and diagonal else 1) if plan.upper else 0
+            if parts:
+                check(self.L.phyloPairsReduceParts(
+                    st, _p(part), _p(plan.part_tiles), plan.ntiles, self.cfg.tile_rows,
+                    self.cfg.tile_cols, _p(plan.rowids), _p(plan.colids), _p(out), plan.ldc,
+                    upper, int(plan.mirror)))
+            else:
+                check(self.L.phyloPairsReduce(
+                    st, _p(part), _p(plan.tiles), plan.ntiles, plan.S, self.cfg.tile_rows,
+                    self.cfg.tile_cols, _p(plan.rowids), _p(plan.colids), _p(out), plan.ldc,
+                    upper, int(plan.mirror)))
         self.launches += 3  # counter fill, pair kernel, reduction
         if diagonal and plan.upper and not plan.diag:
             maxlen = int(np.max(np.diff(a.off[:a.n + 1]))) if a.n else 1

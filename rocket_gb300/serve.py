@@ -39,7 +39,8 @@ import numpy as np
 import torch
 
 from . import _native
-from .engine import Arena, BatchBuilder, EngineConfig, PairEngine, key_limit
+from .engine import (PART_WINDOWS, Arena, BatchBuilder, EngineConfig, PairEngine,
+                     key_limit)
 from .synth import Proteomes
 
 
@@ -296,7 +297,9 @@ class ServingEngine:
         ti = self.cfg.tile_rows
         tj = self.cfg.tile_cols
         tiles = math.ceil(nq / ti) * math.ceil(max(db_n, 1) / tj)
-        parts = tiles * self.cfg.segments * ti * tj * 8.0
+        # a segment's items may run in parts, each with a partial block of its own
+        per_segment = math.ceil(math.ceil(self.db.R / self.cfg.segments) / PART_WINDOWS)
+        parts = tiles * self.cfg.segments * per_segment * ti * tj * 8.0
         out = nq * max(db_n, 1) * 8.0
         return scratch + staged + roff + parts + out
 
