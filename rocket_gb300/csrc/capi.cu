@@ -27,6 +27,7 @@
 #include "cv_build.cuh"
 #include "postings.cuh"
 #include "rank.cuh"
+#include "scan.cuh"
 
 using namespace phylo;
 
@@ -48,37 +49,32 @@ uint64_t single_cand_cap(const BuildGeometry &g, uint64_t max_size) {
     return cap < dense ? cap : dense;
 }
 
-__global__ void k_init_single(BuildArgs a, uint64_t len, uint64_t max_size) {
-    a.seq_off_store[0] = 0;
-    a.seq_off_store[1] = len;
-    a.dst_base[0] = 0;
-    a.dst_cap[0] = max_size;
-}
-
-// arena offsets: vec_off[p] = base + sum of nnz rounded up to 4 entries
-__global__ void k_arena_offsets(const uint64_t *nnz, int B, uint64_t base, uint64_t *vec_off,
-                                uint64_t *dst_base, uint64_t *dst_cap) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        uint64_t off = base;
-        for (int p = 0; p < B; p++) {
+// arena offsets: vec_off[p] = base + sum of nnz rounded up to 4 entries; the padding
+// entries after each vector get key 0xffffffff, value 0.  One CTA.
+constexpr int AO_THREADS = 256;
+__global__ void __launch_bounds__(AO_THREADS) k_arena_offsets(const uint64_t *nnz, int B,
+                                                              uint64_t base, uint64_t *vec_off,
+                                                              uint64_t *dst_base, uint64_t *dst_cap,
+                                                              uint32_t *keys, float *vals) {
+    __shared__ uint64_t sw[AO_THREADS / 32 + 1];
+    uint64_t run = base;
+    for (int p0 = 0; p0 < B; p0 += AO_THREADS) {
+        const int p = p0 + threadIdx.x;
+        const uint64_t n = p < B ? nnz[p] : 0, len = (n + 3) & ~(uint64_t)3;
+        uint64_t tot;
+        const uint64_t off = run + block_excl_scan_u64<AO_THREADS>(len, sw, &tot);
+        run += tot;
+        if (p < B) {
             vec_off[p] = off;
             dst_base[p] = off;
-            dst_cap[p] = nnz[p];
-            off += (nnz[p] + 3) & ~(uint64_t)3;
+            dst_cap[p] = n;
+            for (uint64_t i = off + n; i < off + len; i++) {
+                keys[i] = 0xffffffffu;
+                vals[i] = 0.0f;
+            }
         }
-        vec_off[B] = off;
     }
-}
-
-// padding entries after each vector: key 0xffffffff, value 0
-__global__ void k_arena_pad(const uint64_t *vec_off, const uint64_t *nnz, int B, uint32_t *keys,
-                            float *vals) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= B) return;
-    for (uint64_t i = vec_off[p] + nnz[p]; i < vec_off[p + 1]; i++) {
-        keys[i] = 0xffffffffu;
-        vals[i] = 0.0f;
-    }
+    if (threadIdx.x == 0) vec_off[B] = run;
 }
 
 cudaError_t last_status(uint32_t *d_status, cudaStream_t st, uint32_t *out) {
@@ -152,35 +148,35 @@ int buildCompositionVector(uintptr_t stream, uintptr_t d_temp_storage_ptr, long 
     a.seq_off = a.seq_off_store;
     a.out_keys = (uint32_t *)d_set_keys_ptr;
     a.out_vals = (float *)d_set_values_ptr;
-    k_init_single<<<1, 1, 0, st>>>(a, (uint64_t)string_len, max_size);
-    PHYLO_CHECK(cudaGetLastError());
+    a.single = 1;
+    a.single_len = (uint64_t)string_len;
+    a.single_cap = max_size;
     PHYLO_CHECK(build_plan(a, st));
-    uint64_t nnz = 0;
-    uint32_t status = 0;
-    PHYLO_CHECK(cudaMemcpyAsync(&nnz, a.nnz, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    PHYLO_CHECK(last_status(a.status, st, &status));
-    if (h_size) *h_size = (uint32_t)nnz;
-    if (status & DEV_CAPACITY) {
+    PHYLO_CHECK(build_emit(a, st));  // writes nothing where the checks below fail
+    // one read-back for the whole call: nnz | norm | candidates | status
+    struct {
+        uint64_t nnz;
+        double norm;
+        uint64_t candidates;
+        uint32_t status;
+    } res;
+    PHYLO_CHECK(cudaMemcpyAsync(&res, a.nnz, 28, cudaMemcpyDeviceToHost, st));
+    PHYLO_CHECK(cudaStreamSynchronize(st));
+    if (h_size) *h_size = (uint32_t)res.nnz;
+    if (res.status & DEV_CAPACITY) {
         fprintf(stderr,
                 "error: candidate slots exceed the scratch capacity (%llu) for max_vector_size "
                 "%d\n",
                 (unsigned long long)a.cand_cap, max_vector_size);
         return (int)cudaErrorUnknown;
     }
-    if (nnz > max_size) {
+    if (res.nnz > max_size) {
         fprintf(stderr,
                 "error: size of composition vector (size: %llu) exceeds the given maximum (size: "
                 "%d)\n",
-                (unsigned long long)nnz, max_vector_size);
+                (unsigned long long)res.nnz, max_vector_size);
         return (int)cudaErrorUnknown;
     }
-    PHYLO_CHECK(build_emit(a, st));
-    // padding of the unused tail (native.cu:473-474)
-    if (max_size > nnz) {
-        PHYLO_CHECK(cudaMemsetAsync(a.out_keys + nnz, 0xff, (max_size - nnz) * sizeof(uint32_t), st));
-        PHYLO_CHECK(cudaMemsetAsync(a.out_vals + nnz, 0, (max_size - nnz) * sizeof(float), st));
-    }
-    PHYLO_CHECK(cudaStreamSynchronize(st));
     return (int)cudaGetLastError();
 }
 
@@ -316,13 +312,10 @@ int phyloBuildBatchPlanAsync(uintptr_t stream, uintptr_t d_scratch, long scratch
     a.seq = (const uint8_t *)d_seq;
     a.seq_off = (const uint64_t *)d_seq_off;
     PHYLO_CHECK(build_plan(a, st));
-    // summary layout: int64 nnz[B] | float64 norm[B] | int64 candidates | uint32 status
-    char *h = (char *)h_summary;
-    const size_t B = (size_t)num_proteomes;
-    PHYLO_CHECK(cudaMemcpyAsync(h, a.nnz, 8 * B, cudaMemcpyDeviceToHost, st));
-    PHYLO_CHECK(cudaMemcpyAsync(h + 8 * B, a.norm, 8 * B, cudaMemcpyDeviceToHost, st));
-    PHYLO_CHECK(cudaMemcpyAsync(h + 16 * B, a.cand_total, 8, cudaMemcpyDeviceToHost, st));
-    PHYLO_CHECK(cudaMemcpyAsync(h + 16 * B + 8, a.status, 4, cudaMemcpyDeviceToHost, st));
+    // summary layout, in scratch as in the caller's buffer: int64 nnz[B] | float64 norm[B] |
+    // int64 candidates | uint32 status
+    PHYLO_CHECK(cudaMemcpyAsync(h_summary, a.nnz, 16 * (size_t)num_proteomes + 12,
+                                cudaMemcpyDeviceToHost, st));
     return (int)cudaGetLastError();
 }
 
@@ -352,12 +345,10 @@ int phyloBuildBatchEmit(uintptr_t stream, uintptr_t d_scratch, long scratch_size
     a.out_vals = (float *)d_values;
     a.union_bits = (uint32_t *)d_union_bits;
     uint64_t *vec_off = (uint64_t *)d_vec_off;
-    k_arena_offsets<<<1, 1, 0, st>>>(a.nnz, num_proteomes, (uint64_t)arena_base, vec_off,
-                                     a.dst_base, a.dst_cap);
+    k_arena_offsets<<<1, AO_THREADS, 0, st>>>(a.nnz, num_proteomes, (uint64_t)arena_base, vec_off,
+                                              a.dst_base, a.dst_cap, a.out_keys, a.out_vals);
     PHYLO_CHECK(cudaGetLastError());
     PHYLO_CHECK(build_emit(a, st));
-    k_arena_pad<<<(num_proteomes + 127) / 128, 128, 0, st>>>(vec_off, a.nnz, num_proteomes,
-                                                             a.out_keys, a.out_vals);
     return (int)cudaGetLastError();
 }
 
@@ -396,8 +387,12 @@ static cudaError_t expand_compact_counts(const uint32_t *d_seen, const uint2 *d_
     PHYLO_CHECK(cudaMemcpyAsync(pw.data(), d_pw + (uint64_t)p * nw, sizeof(uint2) * nw,
                                 cudaMemcpyDeviceToHost, st));
     PHYLO_CHECK(cudaStreamSynchronize(st));
-    const uint64_t first = pw[0].x;
-    const uint64_t n = pw[nw - 1].x + (uint64_t)__builtin_popcount(seen[nw - 1]) - first;
+    // ranks are kept for the words that hold seen bits
+    uint64_t first = 0, n = 0;
+    for (uint64_t w = 0; w < nw; w++) {
+        if (n == 0 && seen[w]) first = pw[w].x;
+        n += (uint64_t)__builtin_popcount(seen[w]);
+    }
     if (first + n > cap) return cudaErrorInvalidValue;  // the build ran out of room
     std::vector<uint32_t> cc(n ? n : 1);
     if (n)
@@ -406,7 +401,7 @@ static cudaError_t expand_compact_counts(const uint32_t *d_seen, const uint2 *d_
     PHYLO_CHECK(cudaStreamSynchronize(st));
     memset(h_out, 0, sizeof(uint32_t) * len);
     for (uint64_t w = 0; w < nw; w++) {
-        uint32_t bits = seen[w], r = pw[w].x - (uint32_t)first;
+        uint32_t bits = seen[w], r = bits ? pw[w].x - (uint32_t)first : 0u;
         while (bits) {
             const int j = __builtin_ctz(bits);
             bits &= bits - 1;

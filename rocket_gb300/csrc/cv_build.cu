@@ -15,27 +15,30 @@
 //   into its candidate slot (rank of b in R(m)) -- no sort and no A^K table.
 //
 // Pipeline per batch of proteomes (all kernels take the whole batch):
-//   k_prep          tile bases per proteome
+//   k_begin         zeroed counts, bitmaps and totals; tile bases per proteome
 //   k_count         (K-2)/(K-1) counts, seen (K-1)-mers (the right-extension
 //                   masks are slices of that bitmap), window totals
-//   k_cand_count    candidates per chunk of 2048 (K-1)-mers
-//   scan, k_cand_bases   candidate offsets; proteome p's candidates start at
-//                   cbase[p], a multiple of ALPHA_TILE
-//   k_cand_offsets  per-(K-1)-mer candidate offsets; the key of every candidate
+//   k_cand_count    candidates and seen (K-1)-mers per chunk of bitmap words; in
+//                   further blocks the count -> probability and tuple tables
+//   k_cand_scan     their offsets; proteome p's candidates start at cbase[p], a
+//                   multiple of ALPHA_TILE
+//   k_cand_offsets  per-(K-1)-mer candidate offsets and ranks; the key of every candidate
 //   k_c0_scatter    K-mer counts into candidate slots (zeroed by k_cand_offsets)
 //   k_alpha         Markov alpha (reference double order), flat over the
 //                   candidates: a seen candidate's count is replaced in place by
 //                   its alpha bits (an unseen one keeps count 0: alpha -1);
 //                   survivors counted per segment; norm partials
-//   scan            -> output offset of every segment
-//   k_norm          per-proteome norm, scale, nnz
-//   (host reads nnz, checks capacity)
+//   k_norm          per-proteome norm, scale, nnz, and where each CTA's survivors go
+//   k_tuple_value   the tuples' normalised values
+//   (batches: the host reads nnz)
 //   k_compact       survivors' keys and normalised values, segment by segment
 //   k_union_mark    (with a key bitmap) the candidate keys of every seen (K-1)-mer
 #include "cv_build.cuh"
 #include "hostctx.cuh"
 #include "rank.cuh"
 #include "scan.cuh"
+
+#include <type_traits>
 
 namespace phylo {
 
@@ -89,6 +92,23 @@ __device__ __forceinline__ float markov_alpha(uint32_t full, uint32_t prefix, ui
     return __double2float_rn(__ddiv_rn(__dsub_rn(p, p0), p0));
 }
 
+// alpha from the quotients p = full/n0, pp = prefix/n1, ps = suffix/n1, pm = middle/n2 and
+// ym = RN(1/pm) (see markov_alpha_fast).
+__device__ __forceinline__ float markov_alpha_quot(double p, double pp, double ps, double pm,
+                                                   double ym) {
+    const double a = __dmul_rn(pp, ps);
+    const double q0 = __dmul_rn(a, ym);
+    const double p0 = __fma_rn(__fma_rn(-q0, pm, a), ym, q0);
+    const double d = __dsub_rn(p, p0);
+    if (d == 0.0) return 0.0f;
+    const double y0 = (double)__frcp_rn(__double2float_rn(p0));
+    const double g0 = __dmul_rn(d, y0);
+    const double g1 = __fma_rn(__fma_rn(-g0, p0, d), y0, g0);
+    const long long low = (long long)(__double_as_longlong(g1) & ((1ll << 29) - 1)) - (1ll << 28);
+    if (low <= 256 && low >= -256) return __double2float_rn(__ddiv_rn(d, p0));
+    return __double2float_rn(g1);
+}
+
 // The same alpha with the FP64 work cut down (GB300 issues FP64 at a small
 // fraction of the FP32 rate):
 //   * p, prefix/n1, suffix/n1, middle/n2 come from per-proteome tables holding
@@ -109,24 +129,11 @@ __device__ __forceinline__ float markov_alpha_fast(uint32_t full, uint32_t prefi
     if (n0 == 0u || full >= PROB_TABLE || prefix >= PROB_TABLE || suffix >= PROB_TABLE ||
         middle >= PROB_TABLE)
         return markov_alpha(full, prefix, suffix, middle, n0, n1, n2);
-    const double p = __ldg(&prob[full]);
-    const double pp = __ldg(&prob[PROB_TABLE + prefix]);
-    const double ps = __ldg(&prob[PROB_TABLE + suffix]);
-    const double pm = __ldg(&prob[2 * PROB_TABLE + middle]);
-    const double ym = __ldg(&prob[3 * PROB_TABLE + middle]);
-    const double a = __dmul_rn(pp, ps);
-    const double q0 = __dmul_rn(a, ym);
-    const double p0 = __fma_rn(__fma_rn(-q0, pm, a), ym, q0);
-    const double d = __dsub_rn(p, p0);
-    if (d == 0.0) return 0.0f;
-    const double y0 = (double)__frcp_rn(__double2float_rn(p0));
-    const double g0 = __dmul_rn(d, y0);
-    const double g1 = __fma_rn(__fma_rn(-g0, p0, d), y0, g0);
-    const long long low = (long long)(__double_as_longlong(g1) & ((1ll << 29) - 1)) - (1ll << 28);
-    if (low <= 256 && low >= -256) return __double2float_rn(__ddiv_rn(d, p0));
-    return __double2float_rn(g1);
+    return markov_alpha_quot(__ldg(&prob[full]), __ldg(&prob[PROB_TABLE + prefix]),
+                             __ldg(&prob[PROB_TABLE + suffix]),
+                             __ldg(&prob[2 * PROB_TABLE + middle]),
+                             __ldg(&prob[3 * PROB_TABLE + middle]));
 }
-
 // Sum of non-negative floats as an exact 192-bit fixed-point number in units of
 // 2^-96 (terms below 2^-73 lose their lowest bits; such squares need
 // |alpha| < 2^-36).  Integer addition makes the result independent of order.
@@ -235,49 +242,74 @@ __device__ __forceinline__ uint32_t ext_mask(const BuildArgs &a, int p, uint32_t
 // kernels
 // ---------------------------------------------------------------------------
 
-// prob[p][0][c] = c/n0, [1][c] = c/n1, [2][c] = c/n2, [3][c] = 1/(c/n2): the
-// exact IEEE quotients the reference forms for count c.  grid = (PROB_TABLE/256, B)
-__global__ void k_tables(BuildArgs a) {
-    const int p = blockIdx.y;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= PROB_TABLE) return;
-    const double n0 = (double)a.tot[p * 4 + 0], n1 = (double)a.tot[p * 4 + 1],
-                 n2 = (double)a.tot[p * 4 + 2];
-    double *t = a.prob + (uint64_t)p * 4 * PROB_TABLE;
-    const double pm = __ddiv_rn((double)c, n2);
-    t[c] = __ddiv_rn((double)c, n0);
-    t[PROB_TABLE + c] = __ddiv_rn((double)c, n1);
-    t[2 * PROB_TABLE + c] = pm;
-    t[3 * PROB_TABLE + c] = __ddiv_rn(1.0, pm);
-}
-
-// tile_base[p] = number of TILE-sized tiles of proteomes < p; tile_base[B] = total.
-__global__ void k_prep(int B, const uint64_t *__restrict__ seq_off, uint64_t *tile_base) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        uint64_t acc = 0;
-        for (int p = 0; p < B; p++) {
-            tile_base[p] = acc;
-            acc += div_up(seq_off[p + 1] - seq_off[p], TILE);
+// Zeroes what the counting kernels add to (contiguous in scratch) and the status, and
+// sets tile_base[p] = number of TILE-sized tiles of proteomes < p (tile_base[B] =
+// total) and, for a single proteome, its offsets and output range.
+__global__ void __launch_bounds__(256) k_begin(BuildArgs a) {
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.zero_n8; i += step)
+        a.zero[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.status = 0u;
+        *a.p1_total = 0;
+        if (!a.compact2) *a.p2_total = 0;
+        if (a.single) {
+            a.seq_off_store[0] = 0;
+            a.seq_off_store[1] = a.single_len;
+            a.dst_base[0] = 0;
+            a.dst_cap[0] = a.single_cap;
         }
-        tile_base[B] = acc;
+        uint64_t acc = 0;
+        for (int p = 0; p < a.B; p++) {
+            a.tile_base[p] = acc;
+            acc += div_up(a.single ? a.single_len : a.seq_off[p + 1] - a.seq_off[p], TILE);
+        }
+        a.tile_base[a.B] = acc;
     }
 }
 
-// Alpha of every small count tuple, once per proteome (the same arithmetic as
-// markov_alpha_fast, so a table hit gives the bits the direct path would).
-// grid = (TUPLE_TABLE / 256, B)
-__global__ void k_tuple_alpha(BuildArgs a) {
-    const int p = blockIdx.y;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint32_t)TUPLE_TABLE) return;
+// Blocks of the tables of one proteome (k_cand_count runs them beside its chunks; both
+// need only the totals of k_count).
+constexpr int PROB_BLOCKS = PROB_TABLE / CHUNK_THREADS;
+constexpr int TUPLE_BLOCKS = TUPLE_TABLE / CHUNK_THREADS;
+
+// Block `blk` of proteome p's tables.  prob[p][0][c] = c/n0, [1][c] = c/n1, [2][c] =
+// c/n2, [3][c] = 1/(c/n2): the exact IEEE quotients the reference forms for count c.
+// atab: alpha of every small count tuple, by the same arithmetic, so that a table hit
+// gives the bits the direct path would.
+__device__ void table_block(const BuildArgs &a, int p, int blk) {
+    const uint32_t n0 = a.tot[p * 4 + 0], n1 = a.tot[p * 4 + 1], n2 = a.tot[p * 4 + 2];
+    if (blk < PROB_BLOCKS) {
+        const uint32_t c = blk * CHUNK_THREADS + threadIdx.x;
+        double *t = a.prob + (uint64_t)p * 4 * PROB_TABLE;
+        const double pm = __ddiv_rn((double)c, (double)n2);
+        t[c] = __ddiv_rn((double)c, (double)n0);
+        t[PROB_TABLE + c] = __ddiv_rn((double)c, (double)n1);
+        t[2 * PROB_TABLE + c] = pm;
+        t[3 * PROB_TABLE + c] = __ddiv_rn(1.0, pm);
+        return;
+    }
+    // 256 consecutive tuples: one full, one prefix, two suffixes, every middle
+    static_assert(CHUNK_THREADS == 2 * TUPLE_MID, "a block holds two suffix counts");
+    __shared__ double s_mid[2][TUPLE_MID], s_q[4];
+    const uint32_t t0 = (uint32_t)(blk - PROB_BLOCKS) * CHUNK_THREADS, t = t0 + threadIdx.x;
     const uint32_t mid = t % TUPLE_MID, suf = (t / TUPLE_MID) % TUPLE_PS,
                    pre = (t / (TUPLE_MID * TUPLE_PS)) % TUPLE_PS,
                    full = t / (TUPLE_MID * TUPLE_PS * TUPLE_PS);
-    const uint32_t n0 = a.tot[p * 4 + 0], n1 = a.tot[p * 4 + 1], n2 = a.tot[p * 4 + 2];
+    if (threadIdx.x < TUPLE_MID) {
+        const double pm = __ddiv_rn((double)threadIdx.x, (double)n2);
+        s_mid[0][threadIdx.x] = pm;
+        s_mid[1][threadIdx.x] = __ddiv_rn(1.0, pm);
+    } else if (threadIdx.x < TUPLE_MID + 4) {
+        const int j = threadIdx.x - TUPLE_MID;
+        const uint32_t c = j == 0 ? full : j == 1 ? pre : (t0 / TUPLE_MID + j - 2) % TUPLE_PS;
+        s_q[j] = __ddiv_rn((double)c, (double)(j == 0 ? n0 : n1));
+    }
+    __syncthreads();
     uint32_t bits = 0;
     if (full >= 1 && pre >= 1 && suf >= 1 && mid >= 1 && n0 != 0)
-        bits = __float_as_uint(markov_alpha_fast(full, pre, suf, mid, n0, n1, n2,
-                                                 a.prob + (uint64_t)p * 4 * PROB_TABLE));
+        bits = __float_as_uint(markov_alpha_quot(s_q[0], s_q[1], s_q[2 + threadIdx.x / TUPLE_MID],
+                                                 s_mid[0][mid], s_mid[1][mid]));
     a.atab[(uint64_t)p * TUPLE_TABLE + t] = bits;
 }
 
@@ -389,14 +421,19 @@ __device__ __forceinline__ uint32_t word_candidates(const BuildArgs &a, int p, u
     return s;
 }
 
-// Candidates per chunk of CHUNK_THREADS * wpt bitmap words (wpt consecutive
-// words per thread: 4 for the sparse bitmaps of compact (K-1)-mer tables, else 1).
-// grid = (NCH, B)
+// Candidates and seen (K-1)-mers per chunk of CHUNK_THREADS * wpt bitmap words (wpt
+// consecutive words per thread: 8 for the sparse bitmaps of protein K = 7, else 1).
+// grid = (NCH + table blocks, B).  With compact (K-2)-mer tables also zeroes the entries
+// in use, which k_c0_scatter counts in.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
     const int p = blockIdx.y, c = blockIdx.x;
+    if ((uint64_t)c >= a.NCH) {
+        table_block(a, p, c - (int)a.NCH);
+        return;
+    }
     const uint64_t nw = a.T1s / 32;
     const uint64_t wd0 = ((uint64_t)c * CHUNK_THREADS + threadIdx.x) * a.wpt;
-    uint32_t s = 0;
+    uint32_t s = 0, n = 0;
     for (uint32_t i = 0; i < a.wpt; i++) {
         const uint64_t wd = wd0 + i;
         if (wd >= nw) break;
@@ -404,15 +441,90 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
         const uint32_t sw = bits ? word_candidates(a, p, (uint32_t)(wd * 32), bits) : 0u;
         a.word_cand[(uint64_t)p * nw + wd] = sw;
         s += sw;
+        n += __popc(bits);
     }
     s = __reduce_add_sync(0xffffffffu, s);
-    __shared__ uint32_t ws[CHUNK_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+    n = __reduce_add_sync(0xffffffffu, n);
+    __shared__ uint32_t ws[CHUNK_THREADS / 32], wn[CHUNK_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) {
+        ws[threadIdx.x >> 5] = s;
+        wn[threadIdx.x >> 5] = n;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < CHUNK_THREADS / 32; w++) t += ws[w];
+        uint32_t t = 0, u = 0;
+        for (int w = 0; w < CHUNK_THREADS / 32; w++) {
+            t += ws[w];
+            u += wn[w];
+        }
         a.chunk_cand[(uint64_t)p * a.NCH + c] = t;
+        a.chunk_seen[(uint64_t)p * a.NCH + c] = u;
+    }
+    if (a.compact2) {
+        const uint64_t used = min(*a.p2_total, a.cap2), step = a.NCH * a.B * CHUNK_THREADS;
+        for (uint64_t i = ((uint64_t)p * a.NCH + c) * CHUNK_THREADS + threadIdx.x; i < used;
+             i += step)
+            a.c2[i] = 0u;
+    }
+}
+
+// Exclusive scans of chunk_cand and chunk_seen over the batch, then cbase[p] = start of
+// proteome p's candidates, rounded up to ALPHA_TILE, so that no k_alpha CTA straddles
+// two proteomes.  One CTA: a batch of 24 at K = 6 has 12,000 chunks (two rounds), fewer
+// than the launches of a wider scan cost.
+constexpr int CSCAN_THREADS = 1024, CSCAN_ITEMS = 8;
+__global__ void __launch_bounds__(CSCAN_THREADS) k_cand_scan(BuildArgs a) {
+    __shared__ uint64_t sw[CSCAN_THREADS / 32 + 1];
+    const uint64_t nc = (uint64_t)a.B * a.NCH;
+    uint64_t cand = 0, seen = 0;  // before the round
+    for (uint64_t base = 0; base < nc; base += CSCAN_THREADS * CSCAN_ITEMS) {
+        const uint64_t first = base + (uint64_t)threadIdx.x * CSCAN_ITEMS;
+        uint32_t vc[CSCAN_ITEMS], vs[CSCAN_ITEMS];
+        uint64_t sc = 0, ss = 0, tot;
+#pragma unroll
+        for (int i = 0; i < CSCAN_ITEMS; i++) {
+            vc[i] = first + i < nc ? a.chunk_cand[first + i] : 0u;
+            vs[i] = first + i < nc ? a.chunk_seen[first + i] : 0u;
+            sc += vc[i];
+            ss += vs[i];
+        }
+        uint64_t ec = cand + block_excl_scan_u64<CSCAN_THREADS>(sc, sw, &tot);
+        cand += tot;
+        uint64_t es = seen + block_excl_scan_u64<CSCAN_THREADS>(ss, sw, &tot);
+        seen += tot;
+#pragma unroll
+        for (int i = 0; i < CSCAN_ITEMS; i++) {
+            if (first + i < nc) {
+                a.chunk_cand_off[first + i] = ec;
+                a.chunk_seen_off[first + i] = (uint32_t)es;
+            }
+            ec += vc[i];
+            es += vs[i];
+        }
+    }
+    if (threadIdx.x == 0) a.chunk_cand_off[nc] = cand;
+    __syncthreads();  // the offsets are read back below
+    uint64_t run = 0;
+    for (int p0 = 0; p0 < a.B; p0 += CSCAN_THREADS) {
+        const int p = p0 + threadIdx.x;
+        uint64_t n = 0, tot;
+        if (p < a.B)
+            n = div_up(a.chunk_cand_off[(uint64_t)(p + 1) * a.NCH] -
+                           a.chunk_cand_off[(uint64_t)p * a.NCH], (uint64_t)ALPHA_TILE) * ALPHA_TILE;
+        const uint64_t e = run + block_excl_scan_u64<CSCAN_THREADS>(n, sw, &tot);
+        if (p < a.B) a.cbase[p] = e;
+        run += tot;
+    }
+    if (threadIdx.x == 0) {
+        a.cbase[a.B] = run;
+        *a.cand_total = run;
+        uint32_t full = run > a.cand_cap;
+        if (a.compact1) {
+            *a.p1_total = seen;
+            full |= seen > a.cap1;
+        }
+        if (a.compact2) full |= *a.p2_total > a.cap2;
+        if (full) *a.status = (uint32_t)DEV_CAPACITY;
     }
 }
 
@@ -444,7 +556,9 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t i) {
 // of unseen q are not written); cq = the key q * A + b of every candidate (b over
 // the right-extension mask of q's suffix, ascending), c0a zeroed.  Thread t of
 // the block owns bitmap words [(c * CHUNK_THREADS + t) * wpt, + wpt) and its
-// candidates start at the exclusive scan of the word_cand sums; a warp's 32
+// candidates and seen (K-1)-mers start at the exclusive scans of the word_cand sums and
+// the words' populations (one scan of packed pairs; with compact tables pw1 gets the
+// ranks of the words that hold any); a warp's 32
 // threads own a contiguous run of words and candidates, which the warp
 // processes together: its seen (K-1)-mers, 32 at a time in order (each lane
 // finds its own by a search over the scan of the words' populations), load
@@ -466,12 +580,17 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
     const uint64_t nw = a.T1s / 32;
     const uint32_t *seen = a.seen1 + (uint64_t)p * nw;
     const uint64_t wd0 = ((uint64_t)c * CHUNK_THREADS + threadIdx.x) * a.wpt;
-    uint32_t s = 0;
-    for (uint32_t i = 0; i < a.wpt && wd0 + i < nw; i++) s += a.word_cand[(uint64_t)p * nw + wd0 + i];
+    uint32_t s = 0, npop = 0;
+    for (uint32_t i = 0; i < a.wpt && wd0 + i < nw; i++) {
+        s += a.word_cand[(uint64_t)p * nw + wd0 + i];
+        npop += __popc(seen[wd0 + i]);
+    }
     uint64_t tot;
-    const uint64_t ex = block_excl_scan_u64<CHUNK_THREADS>(s, sw, &tot);
+    const uint64_t ex = block_excl_scan_u64<CHUNK_THREADS>((uint64_t)npop << 32 | s, sw, &tot);
     const uint32_t run0 =
-        (uint32_t)(a.chunk_cand_off[pc] - a.chunk_cand_off[(uint64_t)p * a.NCH] + ex);
+        (uint32_t)(a.chunk_cand_off[pc] - a.chunk_cand_off[(uint64_t)p * a.NCH]) + (uint32_t)ex;
+    // rank of the warp's first seen (K-1)-mer among the batch's
+    uint32_t P = a.chunk_seen_off[pc] + __shfl_sync(0xffffffffu, (uint32_t)(ex >> 32), 0);
     const uint64_t gb = a.cbase[p];
     uint32_t run = __shfl_sync(0xffffffffu, run0, 0);
     const uint32_t r1 = __shfl_sync(0xffffffffu, run0 + s, 31);
@@ -496,9 +615,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
         const uint32_t nseen = __shfl_sync(0xffffffffu, wincl, 31);
         if (nseen == 0u) continue;
         const uint64_t wfirst = wbeg + 32 * t;
-        // compact tables: the rank of the group's first seen (K-1)-mer; the i-th seen
+        // compact tables: P is the rank of the group's first seen (K-1)-mer; the i-th seen
         // (K-1)-mer of the group is then entry P + i
-        const uint64_t P = a.compact1 ? (uint64_t)a.pw1[(uint64_t)p * nw + wfirst].x : 0;
+        if (a.compact1 && wfirst + lane < nw)
+            a.pw1[(uint64_t)p * nw + wfirst + lane] = make_uint2(P + wincl - __popc(wbits), wbits);
         for (uint32_t sb = 0; sb < nseen; sb += 32) {
             const uint32_t i = sb + lane;
             const uint32_t k = warp_owner(wincl, i);
@@ -517,7 +637,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
             // candidate's) and, with compact tables, its count slot (counted by
             // k_c0_scatter)
             if (ok) {
-                const uint64_t qi = a.compact1 ? P + i : c1_index(a, p, q);
+                const uint64_t qi = a.compact1 ? (uint64_t)P + i : c1_index(a, p, q);
                 if (!a.compact1 || qi < a.cap1) {
                     a.coff[qi] = run + cincl - n;
                     if (a.compact1) a.c1[qi] = 0u;
@@ -540,25 +660,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
             __syncwarp();
             run += ctot;
         }
+        P += nseen;
     }
-}
-
-// cbase[p] = start of proteome p's candidates, rounded up to ALPHA_TILE, so that
-// no k_alpha CTA straddles two proteomes.  One thread.
-__global__ void k_cand_bases(BuildArgs a) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint64_t run = 0;
-    for (int p = 0; p < a.B; p++) {
-        a.cbase[p] = run;
-        const uint64_t n =
-            a.chunk_cand_off[(uint64_t)(p + 1) * a.NCH] - a.chunk_cand_off[(uint64_t)p * a.NCH];
-        run += div_up(n, (uint64_t)ALPHA_TILE) * ALPHA_TILE;
-    }
-    a.cbase[a.B] = run;
-    *a.cand_total = run;
-    if (run > a.cand_cap) atomicOr(a.status, (uint32_t)DEV_CAPACITY);
-    if (a.compact1 && *a.p1_total > a.cap1) atomicOr(a.status, (uint32_t)DEV_CAPACITY);
-    if (a.compact2 && *a.p2_total > a.cap2) atomicOr(a.status, (uint32_t)DEV_CAPACITY);
 }
 
 // Every K-window adds one to the slot of its candidate (native.cu:244); with
@@ -666,7 +769,8 @@ constexpr int ALPHA_ILP = 1;  // listed candidates per lane in flight together
 constexpr uint32_t CAND_DROP = 0xffffffffu;
 __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
     __shared__ U192 s_norm[CHUNK_THREADS / 32];
-    __shared__ uint32_t s_m1[CHUNK_THREADS / 32], s_bad[CHUNK_THREADS / 32];
+    __shared__ uint32_t s_m1[CHUNK_THREADS / 32], s_bad[CHUNK_THREADS / 32],
+        s_surv[CHUNK_THREADS / 32];
     __shared__ uint32_t s_lcnt[CHUNK_THREADS / 32][SEG];   // listed candidates: K-mer count,
     __shared__ uint16_t s_lidx[CHUNK_THREADS / 32][SEG];   // index in the segment
     const uint64_t c = blockIdx.x;
@@ -674,15 +778,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t seg = c * (ALPHA_TILE / SEG) + w;
     const uint64_t total = min(*a.cand_total, a.cand_cap);
-    if (g0 >= total) {  // past the last proteome
-        if (lane == 0) a.seg_surv[seg] = 0;
-        if (threadIdx.x == 0) {
-            a.cta_m1[c] = 0;
-            a.cta_bad[c] = 0;
-            a.cta_norm[3 * c] = a.cta_norm[3 * c + 1] = a.cta_norm[3 * c + 2] = 0;
-        }
-        return;
-    }
+    if (g0 >= total) return;  // past the last proteome: k_norm and k_compact stop there too
     const int p = find_owner(a.cbase, a.B, g0);
     const uint32_t np =
         (uint32_t)(a.chunk_cand_off[(uint64_t)(p + 1) * a.NCH] - a.chunk_cand_off[(uint64_t)p * a.NCH]);
@@ -777,17 +873,19 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
         u192_add(acc, o.w0, o.w1, o.w2);
     }
     if (lane == 0) {
-        s_norm[w] = acc; s_m1[w] = m1; s_bad[w] = bad;
+        s_norm[w] = acc; s_m1[w] = m1; s_bad[w] = bad; s_surv[w] = nsurv;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         U192 t = {0, 0, 0};
-        uint32_t tm = 0, tb = 0;
+        uint32_t tm = 0, tb = 0, ts = 0;
         for (int i = 0; i < CHUNK_THREADS / 32; i++) {
             u192_add(t, s_norm[i].w0, s_norm[i].w1, s_norm[i].w2);
             tm += s_m1[i];
             tb |= s_bad[i];
+            ts += s_surv[i];
         }
+        a.cta_surv[c] = ts;
         a.cta_m1[c] = tm;
         a.cta_bad[c] = tb;
         a.cta_norm[3 * c + 0] = t.w0;
@@ -798,25 +896,45 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
 
 // Per proteome: norm = exact sum of the squares rounded once to double
 // (native.cu:415-428 sums the same float squares in double, in CUB's order),
-// scale = sqrt(norm), its reciprocal, nnz, output base.  grid = B, NORM_THREADS
-// threads (the CTA partials of a proteome summed exactly, in any order).
-constexpr int NORM_THREADS = 256;
+// scale = sqrt(norm), its reciprocal, nnz, and cta_out[c] = survivors of the proteome
+// before k_alpha CTA c.  grid = B, NORM_THREADS threads (the CTA partials of a proteome
+// summed exactly, in any order).
+constexpr int NORM_THREADS = 512, NORM_ITEMS = 4;
 __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
     __shared__ U192 s_acc[NORM_THREADS / 32];
-    __shared__ uint64_t s_m1[NORM_THREADS / 32];
+    __shared__ uint64_t s_m1[NORM_THREADS / 32], sw[NORM_THREADS / 32 + 1];
     __shared__ uint32_t s_bad[NORM_THREADS / 32];
     const int p = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t ncta = a.cand_cap / ALPHA_TILE, nseg = a.cand_cap / SEG;
+    const uint64_t ncta = a.cand_cap / ALPHA_TILE;
     const uint64_t c0 = min(a.cbase[p] / ALPHA_TILE, ncta);
     const uint64_t c1 = min(a.cbase[p + 1] / ALPHA_TILE, ncta);
     U192 acc = {0, 0, 0};
-    uint64_t m1 = 0;
+    uint64_t m1 = 0, run = 0;
     uint32_t bad = 0;
-    for (uint64_t c = c0 + threadIdx.x; c < c1; c += NORM_THREADS) {
-        u192_add(acc, a.cta_norm[3 * c], a.cta_norm[3 * c + 1], a.cta_norm[3 * c + 2]);
-        m1 += a.cta_m1[c];
-        bad |= a.cta_bad[c];
+    for (uint64_t base = c0; base < c1; base += NORM_THREADS * NORM_ITEMS) {
+        const uint64_t first = base + (uint64_t)threadIdx.x * NORM_ITEMS;
+        uint32_t v[NORM_ITEMS];
+        uint64_t s = 0, tot;
+#pragma unroll
+        for (int i = 0; i < NORM_ITEMS; i++) {
+            const uint64_t c = first + i;
+            v[i] = 0;
+            if (c < c1) {
+                u192_add(acc, a.cta_norm[3 * c], a.cta_norm[3 * c + 1], a.cta_norm[3 * c + 2]);
+                m1 += a.cta_m1[c];
+                bad |= a.cta_bad[c];
+                v[i] = a.cta_surv[c];
+            }
+            s += v[i];
+        }
+        uint64_t e = run + block_excl_scan_u64<NORM_THREADS>(s, sw, &tot);
+        run += tot;
+#pragma unroll
+        for (int i = 0; i < NORM_ITEMS; i++) {
+            if (first + i < c1) a.cta_out[first + i] = (uint32_t)e;
+            e += v[i];
+        }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -849,10 +967,7 @@ __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
         a.norm[p] = norm;
         a.scale[p] = scale;
         a.rscale[p] = __ddiv_rn(1.0, scale);
-        const uint64_t o0 = a.seg_out_off[min(a.cbase[p] / SEG, nseg)];
-        const uint64_t o1 = a.seg_out_off[min(a.cbase[p + 1] / SEG, nseg)];
-        a.nnz[p] = o1 - o0;
-        a.out_base[p] = o0;
+        a.nnz[p] = run;
     }
 }
 
@@ -889,22 +1004,36 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
 // unseen K-mer (alpha -1); one marked CAND_DROP had alpha 0 and is skipped.  The
 // division by the per-proteome constant scale uses its correctly rounded
 // reciprocal and one FMA correction (Markstein), which yields the correctly
-// rounded double quotient.  grid = cand_cap / ALPHA_TILE
+// rounded double quotient.  grid = cand_cap / ALPHA_TILE, and for a single proteome
+// a.pad_blocks more, which fill the rest of its output with the padding of
+// native.cu:473-474; a single proteome that does not fit leaves its output as it is.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_compact(BuildArgs a) {
     __shared__ uint64_t s_base[SMEM_BASES + 1];
-    const uint64_t c = blockIdx.x, g0 = c * ALPHA_TILE;
+    if (a.single && (*a.status || a.nnz[0] > a.single_cap)) return;
+    const uint64_t c = blockIdx.x, g0 = c * ALPHA_TILE, ncta = a.cand_cap / ALPHA_TILE;
+    if (c >= ncta) {
+        for (uint64_t i = a.nnz[0] + (c - ncta) * CHUNK_THREADS + threadIdx.x; i < a.single_cap;
+             i += (uint64_t)a.pad_blocks * CHUNK_THREADS) {
+            a.out_keys[i] = 0xffffffffu;
+            a.out_vals[i] = 0.0f;
+        }
+        return;
+    }
     if (g0 >= min(*a.cand_total, a.cand_cap)) return;
     const uint64_t *cb = stage_bases(a.cbase, a.B, s_base);
     const int p = find_owner(cb, a.B, g0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t seg = c * (ALPHA_TILE / SEG) + w;
-    if (a.seg_surv[seg] == 0) return;
+    // survivors of the CTA's segments: this warp's come after those of the earlier ones
+    const uint32_t nsurv = lane <= w ? a.seg_surv[c * (ALPHA_TILE / SEG) + lane] : 0u;
+    if (__shfl_sync(0xffffffffu, nsurv, w) == 0) return;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < w ? nsurv : 0u);
     const uint64_t src = seg * SEG;
     const uint32_t np =
         (uint32_t)(a.chunk_cand_off[(uint64_t)(p + 1) * a.NCH] - a.chunk_cand_off[(uint64_t)p * a.NCH]);
     const uint32_t loc0 = (uint32_t)(src - cb[p]);
     const uint32_t nc = loc0 < np ? min((uint32_t)SEG, np - loc0) : 0u;  // its candidates
-    const uint64_t dst = a.dst_base[p] + (a.seg_out_off[seg] - a.out_base[p]);
+    const uint64_t dst = a.dst_base[p] + a.cta_out[c] + before;
     const uint64_t dst_end = a.dst_base[p] + a.dst_cap[p];
     const double scale = a.scale[p];
     const double rs = a.rscale[p];
@@ -984,159 +1113,108 @@ static uint64_t cand_cap_rounded(uint64_t cand_cap) {
     return div_up(cand_cap ? cand_cap : 1, (uint64_t)ALPHA_TILE) * ALPHA_TILE;
 }
 
-size_t build_scratch_bytes(const BuildGeometry &g, int B, uint64_t cand_cap) {
+// One description of the scratch for both its size and its addresses: `take` is called
+// with every array in order.
+template <typename Take>
+static void build_layout(const BuildGeometry &g, int B, uint64_t cand_cap, BuildArgs &r, Take &&take) {
     const uint64_t nc = (uint64_t)B * g.NCH;
     const uint64_t cap = cand_cap_rounded(cand_cap);
     const uint64_t ncta = cap / ALPHA_TILE, nseg = cap / SEG;
+    const uint64_t nw1 = g.T1s / 32 * B, nw2 = g.T2s / 32 * B;
+    const bool compact = compact1_tables(g), compact2 = compact2_tables(g);
+    r.alpha = g.alpha; r.k = g.k; r.A = g.A; r.T1 = g.T1; r.T2 = g.T2; r.NCH = g.NCH; r.B = B;
+    r.wpt = g.wpt;
+    r.T1s = g.T1s;
+    r.T2s = g.T2s;
+    r.fdT2.set((uint32_t)g.T2);
+    r.compact1 = compact ? 1 : 0;
+    r.compact2 = compact2 ? 1 : 0;
+    r.cap1 = compact ? cap : g.T1s * B;
+    r.cap2 = compact2 ? cap : g.T2 * B;
+    r.cand_cap = cap;
+    // zeroed by k_begin: tot up to c1 (dense) or coff
+    take(r.tot, 4 * (uint64_t)B);
+    take(r.seen1, nw1);
+    take(r.seen2, compact2 ? nw2 : 0);
+    if (!compact2) take(r.c2, r.cap2);
+    if (!compact) take(r.c1, r.cap1);
+    take(r.coff, r.cap1);
+    if (compact) take(r.c1, r.cap1);
+    if (compact2) take(r.c2, r.cap2);
+    take(r.pw1, compact ? nw1 : 0);
+    take(r.p1_total, 1);
+    take(r.word_cand, nw1);
+    take(r.pw2, compact2 ? nw2 : 0);
+    take(r.p2_partials, compact2 ? bitmap_prefix_partials(nw2) : 0);
+    take(r.p2_total, 1);
+    take(r.seq_off_store, B + 1);
+    take(r.tile_base, B + 1);
+    take(r.chunk_cand, nc);
+    take(r.chunk_seen, nc);
+    take(r.chunk_cand_off, nc + 1);
+    take(r.chunk_seen_off, nc);
+    take(r.cbase, B + 1);
+    take(r.seg_surv, nseg);
+    take(r.cta_surv, ncta);
+    take(r.cta_out, ncta);
+    take(r.cta_m1, ncta);
+    take(r.cta_norm, 3 * ncta);
+    take(r.cta_bad, ncta);
+    take(r.prob, 4 * (uint64_t)PROB_TABLE * B);
+    take(r.atab, (uint64_t)TUPLE_TABLE * B);
+    take(r.vtab, (uint64_t)TUPLE_TABLE * B);
+    take(r.scale, B);
+    take(r.rscale, B);
+    take(r.dst_base, B);
+    take(r.dst_cap, B);
+    // the results, as the host reads them: nnz[B] | norm[B] | cand_total | status
+    take(r.nnz, 2 * (uint64_t)B + 2);
+    take(r.c0a, cap);
+    take(r.cq, cap);
+}
+
+size_t build_scratch_bytes(const BuildGeometry &g, int B, uint64_t cand_cap) {
+    BuildArgs r;
     size_t s = 0;
-    const bool compact = compact1_tables(g);
-    const uint64_t n1 = compact ? cap : g.T1s * B;  // entries of c1 / coff
-    const uint64_t nw1 = g.T1s / 32 * B;
-    s += scratch_bytes<uint32_t>(n1);              // c1
-    s += scratch_bytes<uint32_t>(n1);              // coff
-    s += scratch_bytes<uint2>(compact ? nw1 : 0);                           // pw1
-    s += scratch_bytes<uint64_t>(compact ? bitmap_prefix_partials(nw1) : 0);  // p1_partials
-    s += scratch_bytes<uint64_t>(1);               // p1_total
-    s += scratch_bytes<uint32_t>(g.T1s / 32 * B);  // seen1
-    s += scratch_bytes<uint32_t>(g.T1s / 32 * B);  // word_cand
-    const bool compact2 = compact2_tables(g);
-    const uint64_t nw2 = g.T2s / 32 * B;
-    s += scratch_bytes<uint32_t>(compact2 ? cap : g.T2 * B);                    // c2
-    s += scratch_bytes<uint32_t>(compact2 ? nw2 : 0);                           // seen2
-    s += scratch_bytes<uint2>(compact2 ? nw2 : 0);                              // pw2
-    s += scratch_bytes<uint64_t>(compact2 ? bitmap_prefix_partials(nw2) : 0);  // p2_partials
-    s += scratch_bytes<uint64_t>(1);                                            // p2_total
-    s += scratch_bytes<uint32_t>(4 * (uint64_t)B); // tot
-    s += scratch_bytes<uint64_t>(B + 1);           // seq_off (single-proteome path)
-    s += scratch_bytes<uint64_t>(B + 1);           // tile_base
-    s += scratch_bytes<uint32_t>(nc);              // chunk_cand
-    s += scratch_bytes<uint64_t>(nc + 1);          // chunk_cand_off
-    s += scratch_bytes<uint64_t>(B + 1);           // cbase
-    s += scratch_bytes<uint64_t>(1);               // cand_total
-    s += scratch_bytes<uint32_t>(nseg);            // seg_surv
-    s += scratch_bytes<uint64_t>(nseg + 1);        // seg_out_off
-    s += scratch_bytes<uint32_t>(ncta);            // cta_m1
-    s += scratch_bytes<uint64_t>(3 * ncta);        // cta_norm
-    s += scratch_bytes<uint32_t>(ncta);            // cta_bad
-    s += scratch_bytes<double>(4 * (uint64_t)PROB_TABLE * B);  // prob tables
-    s += scratch_bytes<uint32_t>((uint64_t)TUPLE_TABLE * B);   // atab
-    s += scratch_bytes<float>((uint64_t)TUPLE_TABLE * B);      // vtab
-    s += scratch_bytes<uint64_t>(scan_temp_bytes(max(nc, nseg) + 1) / 8 + 1);  // scan temp
-    s += scratch_bytes<double>(B);                 // norm
-    s += scratch_bytes<double>(B);                 // scale
-    s += scratch_bytes<double>(B);                 // rscale
-    s += scratch_bytes<uint64_t>(B);               // nnz
-    s += scratch_bytes<uint64_t>(B);               // out_base
-    s += scratch_bytes<uint64_t>(B);               // dst_base
-    s += scratch_bytes<uint64_t>(B);               // dst_cap
-    s += scratch_bytes<uint32_t>(4);               // status
-    s += scratch_bytes<uint32_t>(cap);             // c0a
-    s += scratch_bytes<uint32_t>(cap);             // cq
+    build_layout(g, B, cand_cap, r, [&](auto *&p, uint64_t n) { s += round256(n * sizeof(*p)); });
     return s;
 }
 
 cudaError_t build_carve(const BuildGeometry &g, int B, uint64_t cand_cap, void *scratch,
                         size_t scratch_size, BuildArgs *a) {
     Scratch sc(scratch, scratch_size);
-    const uint64_t nc = (uint64_t)B * g.NCH;
-    const uint64_t cap = cand_cap_rounded(cand_cap);
-    const uint64_t ncta = cap / ALPHA_TILE, nseg = cap / SEG;
     BuildArgs &r = *a;
-    r.alpha = g.alpha; r.k = g.k; r.A = g.A; r.T1 = g.T1; r.T2 = g.T2; r.NCH = g.NCH; r.B = B;
-    r.wpt = g.wpt;
-    r.T1s = g.T1s;
-    const bool compact = compact1_tables(g);
-    const uint64_t n1 = compact ? cap : g.T1s * B;
-    const uint64_t nw1 = g.T1s / 32 * B;
-    r.compact1 = compact ? 1 : 0;
-    r.cap1 = n1;
-    r.c1 = sc.take<uint32_t>(n1);
-    r.coff = sc.take<uint32_t>(n1);
-    r.pw1 = sc.take<uint2>(compact ? nw1 : 0);
-    r.p1_partials = sc.take<uint64_t>(compact ? bitmap_prefix_partials(nw1) : 0);
-    r.p1_total = sc.take<uint64_t>(1);
-    r.seen1 = sc.take<uint32_t>(g.T1s / 32 * B);
-    r.word_cand = sc.take<uint32_t>(g.T1s / 32 * B);
-    const bool compact2 = compact2_tables(g);
-    const uint64_t nw2 = g.T2s / 32 * B;
-    r.compact2 = compact2 ? 1 : 0;
-    r.cap2 = compact2 ? cap : g.T2 * B;
-    r.T2s = g.T2s;
-    r.c2 = sc.take<uint32_t>(r.cap2);
-    r.seen2 = sc.take<uint32_t>(compact2 ? nw2 : 0);
-    r.pw2 = sc.take<uint2>(compact2 ? nw2 : 0);
-    r.p2_partials = sc.take<uint64_t>(compact2 ? bitmap_prefix_partials(nw2) : 0);
-    r.p2_total = sc.take<uint64_t>(1);
-    r.tot = sc.take<uint32_t>(4 * (uint64_t)B);
-    r.seq_off_store = sc.take<uint64_t>(B + 1);
-    r.tile_base = sc.take<uint64_t>(B + 1);
-    r.chunk_cand = sc.take<uint32_t>(nc);
-    r.chunk_cand_off = sc.take<uint64_t>(nc + 1);
-    r.cbase = sc.take<uint64_t>(B + 1);
-    r.cand_total = sc.take<uint64_t>(1);
-    r.seg_surv = sc.take<uint32_t>(nseg);
-    r.seg_out_off = sc.take<uint64_t>(nseg + 1);
-    r.cta_m1 = sc.take<uint32_t>(ncta);
-    r.cta_norm = sc.take<uint64_t>(3 * ncta);
-    r.cta_bad = sc.take<uint32_t>(ncta);
-    r.prob = sc.take<double>(4 * (uint64_t)PROB_TABLE * B);
-    r.atab = sc.take<uint32_t>((uint64_t)TUPLE_TABLE * B);
-    r.vtab = sc.take<float>((uint64_t)TUPLE_TABLE * B);
-    r.fdT2.set((uint32_t)g.T2);
-    r.scan_tmp = sc.take<uint64_t>(scan_temp_bytes(max(nc, nseg) + 1) / 8 + 1);
-    r.norm = sc.take<double>(B);
-    r.scale = sc.take<double>(B);
-    r.rscale = sc.take<double>(B);
-    r.nnz = sc.take<uint64_t>(B);
-    r.out_base = sc.take<uint64_t>(B);
-    r.dst_base = sc.take<uint64_t>(B);
-    r.dst_cap = sc.take<uint64_t>(B);
-    r.status = sc.take<uint32_t>(4);
-    r.c0a = sc.take<uint32_t>(cap);
-    r.cq = sc.take<uint32_t>(cap);
-    r.cand_cap = cap;
-    if (!r.cq) return cudaErrorInvalidValue;  // scratch too small
+    bool ok = true;
+    build_layout(g, B, cand_cap, r, [&](auto *&p, uint64_t n) {
+        p = sc.take<std::remove_reference_t<decltype(*p)>>(n);
+        ok = ok && p;
+    });
+    if (!ok) return cudaErrorInvalidValue;  // scratch too small
+    r.zero = (uint64_t *)r.tot;
+    r.zero_n8 = ((char *)r.coff - (char *)r.tot) / sizeof(uint64_t);
+    r.norm = (double *)(r.nnz + B);
+    r.cand_total = r.nnz + 2 * (uint64_t)B;
+    r.status = (uint32_t *)(r.cand_total + 1);
     return cudaSuccess;
 }
 
 // Phase 1: everything up to per-proteome nnz (no host sync inside).
 cudaError_t build_plan(BuildArgs &a, cudaStream_t st) {
-    const uint64_t nc = (uint64_t)a.B * a.NCH;
-    // dense tables c1 | coff | c2 | tot are contiguous in scratch: zero what needs it
-    if (!a.compact1) PHYLO_CHECK(cudaMemsetAsync(a.c1, 0, sizeof(uint32_t) * a.T1s * a.B, st));
-    PHYLO_CHECK(cudaMemsetAsync(a.seen1, 0, sizeof(uint32_t) * (a.T1s / 32) * a.B, st));
-    if (a.compact2) PHYLO_CHECK(cudaMemsetAsync(a.seen2, 0, sizeof(uint32_t) * (a.T2s / 32) * a.B, st));
-    else PHYLO_CHECK(cudaMemsetAsync(a.c2, 0, sizeof(uint32_t) * a.T2 * a.B, st));
-    PHYLO_CHECK(cudaMemsetAsync(a.tot, 0, sizeof(uint32_t) * 4 * a.B, st));
-    PHYLO_CHECK(cudaMemsetAsync(a.status, 0, sizeof(uint32_t) * 4, st));
-    k_prep<<<1, 32, 0, st>>>(a.B, a.seq_off, a.tile_base);
-    const int grid_seq = device_sm_count() * 8;
-    if (a.compact1) {
-        k_count<true><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
-        PHYLO_CHECK(bitmap_prefix_pairs(a.seen1, a.T1s / 32 * a.B, a.p1_partials, a.pw1,
-                                        a.p1_total, st));
-    } else {
-        k_count<false><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
-        PHYLO_CHECK(cudaMemsetAsync(a.p1_total, 0, sizeof(uint64_t), st));
-    }
-    if (a.compact2) {  // ranks of the seen (K-2)-mers; their counts (k_c0_scatter) start at 0
+    const int sms = device_sm_count();
+    const uint64_t zero_blocks = div_up(a.zero_n8, 4 * 256);
+    k_begin<<<(unsigned)max((uint64_t)1, min(zero_blocks, (uint64_t)sms * 8)), 256, 0, st>>>(a);
+    const int grid_seq = sms * 8;
+    if (a.compact1) k_count<true><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
+    else k_count<false><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
+    if (a.compact2)  // ranks of the seen (K-2)-mers
         PHYLO_CHECK(bitmap_prefix_pairs(a.seen2, a.T2s / 32 * a.B, a.p2_partials, a.pw2,
                                         a.p2_total, st));
-        PHYLO_CHECK(cudaMemsetAsync(a.c2, 0, sizeof(uint32_t) * a.cap2, st));
-    } else {
-        PHYLO_CHECK(cudaMemsetAsync(a.p2_total, 0, sizeof(uint64_t), st));
-    }
-    k_tables<<<dim3(PROB_TABLE / 256, a.B), 256, 0, st>>>(a);
-    k_tuple_alpha<<<dim3(TUPLE_TABLE / 256, a.B), 256, 0, st>>>(a);
-    dim3 gch((unsigned)a.NCH, (unsigned)a.B);
-    k_cand_count<<<gch, CHUNK_THREADS, 0, st>>>(a);
-    PHYLO_CHECK(scan_u32_to_u64(a.chunk_cand, nc, a.chunk_cand_off, a.scan_tmp, st));
-    k_cand_bases<<<1, 32, 0, st>>>(a);
-    k_cand_offsets<<<gch, CHUNK_THREADS, 0, st>>>(a);
+    k_cand_count<<<dim3((unsigned)a.NCH + PROB_BLOCKS + TUPLE_BLOCKS, (unsigned)a.B), CHUNK_THREADS,
+                   0, st>>>(a);
+    k_cand_scan<<<1, CSCAN_THREADS, 0, st>>>(a);
+    k_cand_offsets<<<dim3((unsigned)a.NCH, (unsigned)a.B), CHUNK_THREADS, 0, st>>>(a);
     k_c0_scatter<<<grid_seq, COUNT_THREADS, 0, st>>>(a);
-    const unsigned ncta = (unsigned)(a.cand_cap / ALPHA_TILE);
-    k_alpha<<<ncta, CHUNK_THREADS, 0, st>>>(a);
-    PHYLO_CHECK(scan_u32_to_u64(a.seg_surv, a.cand_cap / SEG, a.seg_out_off, a.scan_tmp, st));
+    k_alpha<<<(unsigned)(a.cand_cap / ALPHA_TILE), CHUNK_THREADS, 0, st>>>(a);
     k_norm<<<a.B, NORM_THREADS, 0, st>>>(a);
     k_tuple_value<<<dim3(TUPLE_TABLE / 256, a.B), 256, 0, st>>>(a);
     return cudaGetLastError();
@@ -1144,18 +1222,20 @@ cudaError_t build_plan(BuildArgs &a, cudaStream_t st) {
 
 // Phase 2: write survivors to out_keys/out_vals at dst_base[p] (capacity dst_cap[p]).
 cudaError_t build_emit(BuildArgs &a, cudaStream_t st) {
-    k_compact<<<(unsigned)(a.cand_cap / ALPHA_TILE), CHUNK_THREADS, 0, st>>>(a);
+    const uint64_t ncta = a.cand_cap / ALPHA_TILE;
+    if (a.single)
+        a.pad_blocks = (unsigned)min(div_up(a.single_cap ? a.single_cap : 1, 8 * CHUNK_THREADS),
+                                     (uint64_t)device_sm_count() * 8);
+    k_compact<<<(unsigned)(ncta + a.pad_blocks), CHUNK_THREADS, 0, st>>>(a);
     if (a.union_bits)
         k_union_mark<<<dim3((unsigned)a.NCH, (unsigned)a.B), CHUNK_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
-// Kernel counting per launch of build_plan + build_emit (for launch accounting).
-// Kernels one batched Plan + Emit launches: plan k_prep, k_count, k_tables,
-// k_tuple_alpha, k_cand_count, scan (3), k_cand_bases, k_cand_offsets,
-// k_c0_scatter, k_alpha, scan (3), k_norm, k_tuple_value; emit
-// k_arena_offsets, k_compact, k_union_mark (with a key bitmap), k_arena_pad.  (Six
-// memsets are not counted.)
-int build_launches_per_batch() { return 17 + 4; }
+// Kernels one batched Plan + Emit launches: plan k_begin, k_count, k_cand_count,
+// k_cand_scan, k_cand_offsets, k_c0_scatter, k_alpha, k_norm, k_tuple_value (and three
+// for the (K-2)-mer ranks of protein K = 7); emit k_arena_offsets, k_compact,
+// k_union_mark (with a key bitmap).
+int build_launches_per_batch() { return 9 + 3; }
 
 }  // namespace phylo

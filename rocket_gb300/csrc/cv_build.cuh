@@ -65,7 +65,7 @@ struct BuildArgs {
     int compact1;
     uint64_t cap1;            // entries of c1 / coff in compact mode
     uint2 *pw1;               // [B * T1s / 32]: {set bits of seen1 before the word, the word}
-    uint64_t *p1_partials, *p1_total;
+    uint64_t *p1_total;
     uint32_t *seen1;          // [B][T1s / 32]: bitmap of the seen (K-1)-mers
     uint32_t *word_cand;      // [B][T1s / 32]: candidates of each bitmap word
     // (K-2)-mer counts: dense [B][T2], or, when `compact2` (beyond 2^20 entries),
@@ -79,16 +79,18 @@ struct BuildArgs {
     uint32_t *tot;            // [B][4]: n0, n1, n2, -
     // per (proteome, chunk of CH (K-1)-mers)
     uint32_t *chunk_cand;     // candidates per chunk
-    uint64_t *chunk_cand_off; // exclusive scan (global over the batch), [nc+1]
+    uint32_t *chunk_seen;     // seen (K-1)-mers per chunk
+    uint64_t *chunk_cand_off; // exclusive scans (global over the batch), [nc+1]
+    uint32_t *chunk_seen_off; // [nc]
     // candidate index space: proteome p owns [cbase[p], cbase[p+1]), cbase[p] a
     // multiple of ALPHA_TILE; cbase[B] = *cand_total
     uint64_t *cbase;          // [B+1]
     uint64_t *cand_total;     // [1]
     uint32_t *cq;             // [cand_cap]: the key of each candidate, then of each survivor
-    // per segment of SEG candidates (survivors compacted to the segment's start)
-    uint32_t *seg_surv;       // [nseg]
-    uint64_t *seg_out_off;    // exclusive scan, [nseg+1]
+    uint32_t *seg_surv;       // [nseg] survivors per segment of SEG candidates
     // per CTA of k_alpha (ALPHA_TILE candidates)
+    uint32_t *cta_surv;       // survivors
+    uint32_t *cta_out;        // survivors of the proteome before the CTA
     uint32_t *cta_m1;         // survivors with alpha^2 == 1
     uint64_t *cta_norm;       // [ncta][3]: sum of the other alpha^2 as 192-bit fixed point, 2^-96 units
     uint32_t *cta_bad;        // bit 0 a NaN square, bit 1 an infinite one
@@ -96,12 +98,19 @@ struct BuildArgs {
     uint32_t *atab;           // [B][TUPLE_TABLE]: alpha bits of each count tuple
     float *vtab;              // [B][TUPLE_TABLE]: float(alpha / sqrt(norm)) of each tuple
     FastDiv fdT2;             // division by A^(K-2)
-    uint64_t *scan_tmp;
     // per proteome results
     double *norm, *scale, *rscale;  // sum alpha^2, sqrt of it, RN(1/sqrt)
-    uint64_t *nnz, *out_base;
+    uint64_t *nnz;
     uint64_t *dst_base, *dst_cap;  // where k_compact writes proteome p
     uint32_t *status;
+    // what k_begin zeroes
+    uint64_t *zero;
+    uint64_t zero_n8;
+    // a single proteome (the drop-in call): its length and output capacity, which
+    // k_compact pads to
+    int single;
+    uint64_t single_len, single_cap;
+    unsigned pad_blocks;
     // K-mer counts per candidate, replaced by alpha bits
     uint32_t *c0a;
     uint64_t cand_cap;
