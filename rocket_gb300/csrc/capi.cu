@@ -375,10 +375,11 @@ int phyloBuildBatchNorms(uintptr_t stream, uintptr_t d_scratch, long scratch_siz
 // Dense (K-1)- and (K-2)-mer count tables and n0/n1/n2 of proteome p of the last
 // Plan (for count-parity checks).  Synchronous.
 // Compact count table of proteome p (entry pw[w].x + rank of the bit in word w for
-// every set bit of the seen bitmap's nw words) expanded into a dense host table of
-// `len` entries.
+// every set bit of the seen bitmap's nw words; its count is the first of its `stride`
+// words) expanded into a dense host table of `len` entries.
 static cudaError_t expand_compact_counts(const uint32_t *d_seen, const uint2 *d_pw,
-                                         const uint32_t *d_counts, uint64_t cap, uint64_t nw,
+                                         const uint32_t *d_counts, int stride, uint64_t cap,
+                                         uint64_t nw,
                                          int p, uint64_t len, uint32_t *h_out, cudaStream_t st) {
     std::vector<uint32_t> seen(nw);
     std::vector<uint2> pw(nw);
@@ -394,9 +395,9 @@ static cudaError_t expand_compact_counts(const uint32_t *d_seen, const uint2 *d_
         n += (uint64_t)__builtin_popcount(seen[w]);
     }
     if (first + n > cap) return cudaErrorInvalidValue;  // the build ran out of room
-    std::vector<uint32_t> cc(n ? n : 1);
+    std::vector<uint32_t> cc(n ? n * stride : 1);
     if (n)
-        PHYLO_CHECK(cudaMemcpyAsync(cc.data(), d_counts + first, sizeof(uint32_t) * n,
+        PHYLO_CHECK(cudaMemcpyAsync(cc.data(), d_counts + first * stride, sizeof(uint32_t) * n * stride,
                                     cudaMemcpyDeviceToHost, st));
     PHYLO_CHECK(cudaStreamSynchronize(st));
     memset(h_out, 0, sizeof(uint32_t) * len);
@@ -405,7 +406,7 @@ static cudaError_t expand_compact_counts(const uint32_t *d_seen, const uint2 *d_
         while (bits) {
             const int j = __builtin_ctz(bits);
             bits &= bits - 1;
-            if (w * 32 + j < len) h_out[w * 32 + j] = cc[r];
+            if (w * 32 + j < len) h_out[w * 32 + j] = cc[(size_t)r * stride];
             r++;
         }
     }
@@ -426,13 +427,13 @@ int phyloBuildBatchCounts(uintptr_t stream, uintptr_t d_scratch, long scratch_si
                             (size_t)scratch_size, &a));
     cudaStream_t st = (cudaStream_t)stream;
     if (a.compact1) {
-        PHYLO_CHECK(expand_compact_counts(a.seen1, a.pw1, a.c1, a.cap1, g.T1s / 32, p, g.T1, h_c1, st));
+        PHYLO_CHECK(expand_compact_counts(a.seen1, a.pw1, (const uint32_t *)a.cc, 2, a.cap1, g.T1s / 32, p, g.T1, h_c1, st));
     } else {
         PHYLO_CHECK(cudaMemcpyAsync(h_c1, a.c1 + (uint64_t)p * g.T1s, sizeof(uint32_t) * g.T1,
                                     cudaMemcpyDeviceToHost, st));
     }
     if (a.compact2) {
-        PHYLO_CHECK(expand_compact_counts(a.seen2, a.pw2, a.c2, a.cap2, g.T2s / 32, p, g.T2, h_c2, st));
+        PHYLO_CHECK(expand_compact_counts(a.seen2, a.pw2, a.c2, 1, a.cap2, g.T2s / 32, p, g.T2, h_c2, st));
     } else {
         PHYLO_CHECK(cudaMemcpyAsync(h_c2, a.c2 + (uint64_t)p * g.T2, sizeof(uint32_t) * g.T2,
                                     cudaMemcpyDeviceToHost, st));

@@ -23,7 +23,8 @@
 //   k_cand_scan     their offsets; proteome p's candidates start at cbase[p], a
 //                   multiple of ALPHA_TILE
 //   k_cand_offsets  per-(K-1)-mer candidate offsets and ranks; the key of every candidate
-//   k_c0_scatter    K-mer counts into candidate slots (zeroed by k_cand_offsets)
+//   k_c0_scatter    (K-1)-mer counts (compact tables) and K-mer counts into candidate
+//                   slots (zeroed by k_cand_offsets)
 //   k_alpha         Markov alpha (reference double order), flat over the
 //                   candidates: a seen candidate's count is replaced in place by
 //                   its alpha bits (an unseen one keeps count 0: alpha -1);
@@ -215,6 +216,10 @@ __device__ __forceinline__ uint64_t c1_index(const BuildArgs &a, int p, uint32_t
     if (!a.compact1) return (uint64_t)p * a.T1s + q;
     const uint2 t = __ldg(&a.pw1[(uint64_t)p * (a.T1s / 32) + (q >> 5)]);  // {prefix, seen word}
     return (uint64_t)t.x + (uint32_t)__popc(t.y & ((1u << (q & 31u)) - 1u));
+}
+
+__device__ __forceinline__ uint32_t c1_load(const BuildArgs &a, uint64_t i) {
+    return a.compact1 ? __ldg(&a.cc[i].x) : __ldg(&a.c1[i]);
 }
 
 // Index of (K-2)-mer m of proteome p in c2: dense row entry, or its rank among
@@ -639,8 +644,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
             if (ok) {
                 const uint64_t qi = a.compact1 ? (uint64_t)P + i : c1_index(a, p, q);
                 if (!a.compact1 || qi < a.cap1) {
-                    a.coff[qi] = run + cincl - n;
-                    if (a.compact1) a.c1[qi] = 0u;
+                    if (a.compact1) a.cc[qi] = make_uint2(0u, run + cincl - n);
+                    else a.coff[qi] = run + cincl - n;
                 }
             }
             // their candidate keys: each lane writes its own (at most A) into the warp's
@@ -668,8 +673,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
 // compact (K-1)-mer tables every (K-1)-window also adds one to its count.  A
 // thread's windows go through the dependent steps together (codes, rank loads,
 // counts, offsets and masks, slot atomics), so their loads are in flight at once.
-// The L2 atomics, not those loads, set the pace: the same kernel with four windows
-// per thread instead of two measured no faster.
+// The L2 requests, not the latency of the loads, set the pace: four windows per thread
+// instead of two measured no faster, and one 64-bit atomic for count and offset instead
+// of an atomic and a load took the build of 200 uneven proteomes from 22.2 to 21.0 ms.
 __global__ void __launch_bounds__(COUNT_THREADS) k_c0_scatter(BuildArgs a) {
     __shared__ uint8_t dig[TILE + 16];
     const int K = a.k;
@@ -727,14 +733,15 @@ __global__ void __launch_bounds__(COUNT_THREADS) k_c0_scatter(BuildArgs a) {
             if (mi[u] < a.cap2) atomicAdd(&a.c2[mi[u]], 1u);
             if (wi[u] != ~0ull) {
                 const bool in_cap = !a.compact1 || wi[u] < a.cap1;
-                if (a.compact1 && in_cap) atomicAdd(&a.c1[wi[u]], 1u);
+                if (a.compact1 && in_cap)
+                    co[u] = (uint32_t)(atomicAdd((unsigned long long *)&a.cc[wi[u]], 1ull) >> 32);
                 if (!in_cap || bd[u] == 0xffu) wi[u] = ~0ull;
             }
         }
 #pragma unroll
         for (int u = 0; u < NU; u++) {
             if (wi[u] != ~0ull) {
-                co[u] = __ldg(&a.coff[wi[u]]);
+                if (!a.compact1) co[u] = __ldg(&a.coff[wi[u]]);
                 em[u] = ext_mask(a, p, a.fdT2.mod(w[u]));
             }
         }
@@ -828,10 +835,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
             const uint32_t b = key[j] - q * A;
             const uint32_t m = a.fdT2.mod(q);
             const bool seen = ok && full[j] != 0u;
-            pre[j] = seen ? __ldg(&a.c1[c1_index(a, p, q)]) : 0u;
+            pre[j] = seen ? c1_load(a, c1_index(a, p, q)) : 0u;
             const uint64_t mi = seen ? c2_index(a, p, m) : 0;
             mid[j] = seen && (!a.compact2 || mi < a.cap2) ? __ldg(&a.c2[mi]) : 0u;
-            suf[j] = seen ? __ldg(&a.c1[c1_index(a, p, m * A + b)]) : 0u;
+            suf[j] = seen ? c1_load(a, c1_index(a, p, m * A + b)) : 0u;
         }
 #pragma unroll
         for (int j = 0; j < ALPHA_ILP; j++) {
@@ -1004,7 +1011,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
 // unseen K-mer (alpha -1); one marked CAND_DROP had alpha 0 and is skipped.  The
 // division by the per-proteome constant scale uses its correctly rounded
 // reciprocal and one FMA correction (Markstein), which yields the correctly
-// rounded double quotient.  grid = cand_cap / ALPHA_TILE, and for a single proteome
+// rounded double quotient.  Most segments drop nothing and move as they are, eight
+// entries per lane in flight; the others place theirs by ballots, at three times the
+// instructions (with ballots throughout, 62% of the issue slots: 200 uneven proteomes
+// 22.2 -> 21.7 ms).  grid = cand_cap / ALPHA_TILE, and for a single proteome
 // a.pad_blocks more, which fill the rest of its output with the padding of
 // native.cu:473-474; a single proteome that does not fit leaves its output as it is.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_compact(BuildArgs a) {
@@ -1040,6 +1050,33 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_compact(BuildArgs a) {
     const float *vtab = a.vtab + (uint64_t)p * TUPLE_TABLE;
     const bool finite = isfinite(scale) && scale > 0.0;
     const float vm1 = __double2float_rn(-rs);  // RN(-1/scale) == -RN(1/scale)
+    auto value = [&](uint32_t b) {
+        if (b == 0u) return vm1;  // unseen K-mer: alpha -1
+        if ((b & TUPLE_TAG) == TUPLE_TAG) return __ldg(&vtab[b & ~TUPLE_TAG]);
+        const float f = __uint_as_float(b);
+        if (!finite || !isfinite(f)) return __double2float_rn(__ddiv_rn((double)f, scale));
+        return f == -1.0f ? vm1 : div_by_scale(f, scale, rs);
+    };
+    if (__shfl_sync(0xffffffffu, nsurv, w) == nc && dst + nc <= dst_end) {
+        // nothing dropped: the segment moves as it is
+        constexpr int V = SEG / 32;
+        uint32_t bits[V], key[V];
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            const uint32_t i = 32 * u + lane;
+            bits[u] = i < nc ? a.c0a[src + i] : 0u;
+            key[u] = i < nc ? a.cq[src + i] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            const uint32_t i = 32 * u + lane;
+            if (i < nc) {
+                a.out_keys[dst + i] = key[u];
+                a.out_vals[dst + i] = value(bits[u]);
+            }
+        }
+        return;
+    }
     // four candidates per lane in flight: loads first, then the stores
     constexpr int U = 4;
     uint32_t out = 0;  // survivors written so far
@@ -1056,17 +1093,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_compact(BuildArgs a) {
             const bool surv = bits[u] != CAND_DROP;
             const unsigned bal = __ballot_sync(0xffffffffu, surv);
             if (surv) {
-                float v;
-                if (bits[u] == 0u) {
-                    v = vm1;  // unseen K-mer: alpha -1
-                } else if ((bits[u] & TUPLE_TAG) == TUPLE_TAG) {
-                    v = __ldg(&vtab[bits[u] & ~TUPLE_TAG]);
-                } else {
-                    const float f = __uint_as_float(bits[u]);
-                    if (!finite || !isfinite(f)) v = __double2float_rn(__ddiv_rn((double)f, scale));
-                    else if (f == -1.0f) v = vm1;
-                    else v = div_by_scale(f, scale, rs);
-                }
+                const float v = value(bits[u]);
                 const uint64_t o = dst + out + __popc(bal & ((1u << lane) - 1u));
                 if (o < dst_end) {
                     a.out_keys[o] = key[u];
@@ -1138,8 +1165,8 @@ static void build_layout(const BuildGeometry &g, int B, uint64_t cand_cap, Build
     take(r.seen2, compact2 ? nw2 : 0);
     if (!compact2) take(r.c2, r.cap2);
     if (!compact) take(r.c1, r.cap1);
-    take(r.coff, r.cap1);
-    if (compact) take(r.c1, r.cap1);
+    take(r.coff, compact ? 0 : r.cap1);
+    take(r.cc, compact ? r.cap1 : 0);
     if (compact2) take(r.c2, r.cap2);
     take(r.pw1, compact ? nw1 : 0);
     take(r.p1_total, 1);

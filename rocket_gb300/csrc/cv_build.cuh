@@ -60,10 +60,13 @@ struct BuildArgs {
     uint64_t *tile_base;      // [B+1]
     // (K-1)-mer tables: dense [B][T1s] (coff written for seen (K-1)-mers only), or,
     // when `compact1` (tables beyond 2^20 entries), one entry per seen (K-1)-mer of
-    // the batch, at its rank among the seen bits: pw1[word].x + popc(bits below)
-    uint32_t *c1, *coff;
+    // the batch, at its rank among the seen bits: pw1[word].x + popc(bits below), with
+    // the count and the offset together, so that k_c0_scatter's one atomic per window
+    // adds to the count and returns the offset
+    uint32_t *c1, *coff;      // dense
+    uint2 *cc;                // compact: {count, coff}
     int compact1;
-    uint64_t cap1;            // entries of c1 / coff in compact mode
+    uint64_t cap1;            // entries of c1 and coff, or of cc
     uint2 *pw1;               // [B * T1s / 32]: {set bits of seen1 before the word, the word}
     uint64_t *p1_total;
     uint32_t *seen1;          // [B][T1s / 32]: bitmap of the seen (K-1)-mers
