@@ -841,20 +841,20 @@ cudaError_t range_index_launch(const uint32_t *keys, const uint64_t *vec_off, ui
 // reduction of partial blocks
 // ---------------------------------------------------------------------------
 
-// grid = (ntiles, tile rows), block = (tile columns, AP_RED): one (row, column) pair per
-// threadIdx.x, its partials split evenly over threadIdx.y; each share is summed in
-// part order and the shares in order (double-double), so the result does not depend on
-// how the items were scheduled.  Bound by the latency of a pair's chain of partials, so
-// the chain is cut in AP_RED (one thread per pair: 107 us for 8 tiles of 152 partial
-// blocks, 128 uniform proteomes).
-constexpr int AP_RED = 4;
-__global__ void __launch_bounds__(256 * AP_RED) k_ap_reduce(ApReduceArgs r) {
-    __shared__ DD s_acc[AP_RED - 1][256];
+// grid = (ntiles, tile rows, tile columns / 32), block = (32, AP_RED): one (row, column)
+// pair per threadIdx.x, its partials split evenly over threadIdx.y; each share is
+// summed in part order and the shares in order (double-double), so the result does not
+// depend on how the items were scheduled.  Bound by the latency of a pair's chain of
+// partials, so the chain is cut in AP_RED (with one thread per pair 107 us for 8 tiles of
+// 152 partial blocks, 128 uniform proteomes; with four 79 us for one tile of 348).
+constexpr int AP_RED = 16;
+__global__ void __launch_bounds__(32 * AP_RED) k_ap_reduce(ApReduceArgs r) {
+    __shared__ DD s_acc[AP_RED - 1][32];
     const uint32_t *t = r.tiles + (uint64_t)blockIdx.x * r.tile_words;
     const uint32_t row0 = t[0], nrow = t[1], col0 = t[2], ncol = t[3];
     const uint64_t part0 = r.tile_words == 8 ? t[4] : (uint64_t)blockIdx.x * r.S;
     const uint32_t S = r.tile_words == 8 ? t[5] : r.S;
-    const uint32_t c = threadIdx.x, i = blockIdx.y, y = threadIdx.y;
+    const uint32_t c = blockIdx.z * 32 + threadIdx.x, i = blockIdx.y, y = threadIdx.y;
     const uint32_t rowpos = row0 + i, colpos = col0 + c;
     bool use = c < ncol && i < nrow;
     if (r.upper == 1 && !(rowpos < colpos)) use = false;
@@ -871,12 +871,12 @@ __global__ void __launch_bounds__(256 * AP_RED) k_ap_reduce(ApReduceArgs r) {
             dd_add(acc, (double)p.hi);
             dd_add(acc, (double)p.lo);
         }
-        if (y) s_acc[y - 1][c] = acc;
+        if (y) s_acc[y - 1][threadIdx.x] = acc;
     }
     __syncthreads();
     if (!use || y) return;
 #pragma unroll
-    for (int k = 0; k < AP_RED - 1; k++) acc = dd_merge(acc, s_acc[k][c]);
+    for (int k = 0; k < AP_RED - 1; k++) acc = dd_merge(acc, s_acc[k][threadIdx.x]);
     const double v = __dadd_rn(acc.hi, acc.lo);
     const uint32_t rowid = r.rowids[rowpos], colid = r.colids[colpos];
     r.out[(uint64_t)rowid * r.ldc + colid] = v;
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(256 * AP_RED) k_ap_reduce(ApReduceArgs r) {
 
 cudaError_t ap_reduce_launch(const ApReduceArgs &r, cudaStream_t st) {
     if (r.ntiles == 0) return cudaSuccess;
-    k_ap_reduce<<<dim3(r.ntiles, r.ti), dim3(r.tj, AP_RED), 0, st>>>(r);
+    k_ap_reduce<<<dim3(r.ntiles, r.ti, r.tj / 32), dim3(32, AP_RED), 0, st>>>(r);
     return cudaGetLastError();
 }
 
