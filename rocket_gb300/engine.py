@@ -64,25 +64,25 @@ def auto_tile_cols(n_cols: int) -> int:
     return 256 if n_cols >= 384 else 128
 
 
-def split_segments(windows: np.ndarray, est: np.ndarray, tail: np.ndarray, grid: int,
-                   most: int) -> np.ndarray:
+def split_segments(windows: np.ndarray, cost: np.ndarray, tail: np.ndarray, count: int,
+                   grid: int, most: int) -> np.ndarray:
     """Parts per segment of a window plan with too few segments to fill the GPU.  A part
     is computed by a CTA of its own with the sums the whole segment would form
-    (phyloPairsLaunchParts).  ``windows``: windows of each segment; ``est``: its cost;
-    ``tail``: windows a part goes on past its own to finish its lanes' FP32 runs.  Of
-    several totals up to ``most`` items, the one whose items, PART_SETUP windows and a
-    tail longer than their share, finish first on ``grid`` CTAs, longest first."""
+    (phyloPairsLaunchParts).  Per tile, ``windows`` of its segments, their ``cost`` and
+    ``tail``, the windows a part goes on past its own to finish its lanes' FP32 runs;
+    ``count`` segments per tile.  Of several totals up to ``most`` items, the one that
+    finishes first on ``grid`` CTAs: the work of all items, each with PART_SETUP windows
+    (and a tail) on top, shared evenly, and the longest item to wait for."""
     best, best_time = None, math.inf
-    total = est.sum()
-    for goal in (0, 1, 2, 4, most / grid):
-        n = np.ceil(est * (goal * grid / total)) if goal else np.ones(len(est))
-        n = np.clip(n, 1, windows).astype(np.int64)
-        extra = np.where(n > 1, PART_SETUP + tail, PART_SETUP)
-        cost = np.sort(np.repeat(est * (1.0 / n + extra / windows), n))[::-1]
-        time = cost[::grid].sum()
+    share = cost * (grid / (count * cost.sum()))
+    unit = cost / windows
+    for goal in (0.0, 1.0, 2.0, 4.0, most / grid):
+        n = np.minimum(np.maximum(np.ceil(share * goal), 1.0), windows)
+        item = unit * (windows / n + PART_SETUP + np.where(n > 1, tail, 0.0))
+        time = count * (item * n).sum() / grid + item.max()
         if time < best_time:
             best, best_time = n, time
-    return best
+    return best.astype(np.int64)
 
 
 # --------------------------------------------------------------------------
@@ -233,8 +233,11 @@ class BatchBuilder:
     def _build_into(self, arena: Arena, seq: torch.Tensor, seq_off: np.ndarray, lens: np.ndarray,
                     stream: torch.cuda.Stream, host: Optional[torch.Tensor] = None) -> None:
         n = len(seq_off) - 1
-        d_seq_off_all = torch.from_numpy(seq_off).to(self.device, non_blocking=False)
         batches = [(f, min(self.max_batch, n - f)) for f in range(0, n, self.max_batch)]
+        # every batch's offsets from its own first residue, in one copy
+        rel = [seq_off[f:f + b + 1] - seq_off[f] for f, b in batches]
+        d_rel = torch.from_numpy(np.concatenate(rel or [np.zeros(1, np.int64)])).to(self.device)
+        rel_at = np.cumsum([0] + [len(x) for x in rel])
         if host is not None and len(batches) == 1:  # nothing to overlap: one copy, in order
             seq[:int(seq_off[-1])].copy_(host[:int(seq_off[-1])], non_blocking=True)
             host = None
@@ -253,14 +256,18 @@ class BatchBuilder:
             start.record(stream)
             self._side.wait_event(start)
             streams.append(self._side)
-        keep = []  # device tensors used by queued work, held until the build is joined
+        per = np.minimum(8 * lens + 65536, key_limit(self.alphabet, self.k))
+        cands = [int(per[f:f + b].sum()) for f, b in batches]
+        for slot, st in enumerate(streams):  # scratch for the largest batch of each stream
+            with torch.cuda.stream(st):
+                for bi in sorted(range(slot, len(batches), len(streams)), key=lambda i: -cands[i]):
+                    self._scratch_for(slot, batches[bi][1], cands[bi])
 
         def enqueue(bi: int) -> dict:
             first, B = batches[bi]
             slot = bi % len(streams)
             st = streams[slot]
-            lens_b = lens[first:first + B]
-            cand = int(np.sum(np.minimum(8 * lens_b + 65536, key_limit(self.alphabet, self.k))))
+            cand = cands[bi]
             base = int(seq_off[first])
             end = int(seq_off[first + B])
             if host is not None and end > base:  # this batch's residues, ahead of its build
@@ -269,11 +276,9 @@ class BatchBuilder:
                 copied = torch.cuda.Event()
                 copied.record(self._copy)
                 st.wait_event(copied)
-            with torch.cuda.stream(st):
-                d_off = d_seq_off_all[first:first + B + 1] - base
-                scr = self._scratch_for(slot, B, cand)
+            scr = self._scratch_for(slot, B, cand)
+            d_off = d_rel[int(rel_at[bi]):int(rel_at[bi + 1])]
             d_seq = seq[base:end]
-            keep.append(d_off)
             summ = self._summary_for(slot)
             check(self.L.phyloBuildBatchPlanAsync(
                 int(st.cuda_stream), _p(scr), scr.numel(), self.alphabet.encode(), self.k, B,
@@ -359,9 +364,8 @@ class BatchBuilder:
             done = torch.cuda.Event()
             done.record(self._side)
             stream.wait_event(done)
-            # tensors the side stream used stay alive until it has finished with them
-            for t in keep:
-                t.record_stream(self._side)
+            # the offsets stay alive until the side stream has finished with them
+            d_rel.record_stream(self._side)
 
 
 def upload_proteomes(data: np.ndarray, device=None, pinned: Optional[torch.Tensor] = None,
@@ -673,65 +677,79 @@ class PairEngine:
         item_tile = t_of[order]
         share = share[order]
         dev = self.device
+        parts = part_tiles = np.zeros((0, 0), np.int64)
         cut = None
         if self.cfg.algorithm == "window" and self.cfg.tile_rows == AP_TI and \
                 self.cfg.tile_cols >= 128:
-            cut = self._cut_items(items, est, host_tiles, col_nnz[colids])
+            cut = self._cut_items(S, cost, host_tiles, col_nnz[colids])
             if cut is not None:
-                nparts = len(cut[0])
+                parts, part_tiles = cut
+                nparts = len(parts)
+        # one copy to the device: each array from a 16-byte boundary
+        arrays = [rowids, colids, host_tiles, items, parts, part_tiles]
+        ends = np.cumsum([-(-x.size // 4) * 4 for x in arrays])
+        flat = np.zeros(int(ends[-1]), np.int32)
+        for x, e in zip(arrays, ends):
+            flat[e - (-(-x.size // 4) * 4):][:x.size] = x.ravel()
+        on_dev = torch.from_numpy(flat).to(dev)
+        views = [on_dev[e - (-(-x.size // 4) * 4):][:x.size].view(x.shape)
+                 for x, e in zip(arrays, ends)]
         plan = PairPlan(
-            rowids=torch.from_numpy(rowids.astype(np.int32)).to(dev),
-            colids=torch.from_numpy(colids.astype(np.int32)).to(dev),
-            tiles=torch.from_numpy(host_tiles.astype(np.int32)).to(dev),
-            items=torch.from_numpy(items.astype(np.int32)).to(dev),
+            rowids=views[0], colids=views[1], tiles=views[2], items=views[3],
             ntiles=ntiles, nitems=len(items), S=S, upper=upper, mirror=mirror, ldc=ldc,
             est=est, pairs=pairs, host_items=items, algorithm=self.cfg.algorithm,
             nparts=nparts, host_rowids=rowids, host_colids=colids, host_tiles=host_tiles,
             item_tile=item_tile, item_share=share)
         if cut is not None:
             plan.host_parts, plan.host_part_tiles = cut
-            plan.parts = torch.from_numpy(plan.host_parts.astype(np.int32)).to(dev)
-            plan.part_tiles = torch.from_numpy(plan.host_part_tiles.astype(np.int32)).to(dev)
+            plan.parts, plan.part_tiles = views[4], views[5]
         return plan
 
-    def _cut_items(self, items, est, host_tiles, nnz_of_col):
-        """(parts [n, 12], tiles [ntiles, 8]) of a plan whose items are too few to fill the
-        GPU, longest first, or None where no item is cut.  ``items`` in launch order;
-        ``nnz_of_col``: entries of the plan's columns in their order, most first."""
+    def _cut_items(self, S, cost, host_tiles, nnz_of_col):
+        """(parts [n, 12], tiles [ntiles, 8]) of a plan of S segments per tile whose items
+        are too few to fill the GPU, longest first, or None where no segment is cut.
+        ``cost``: of each tile; ``nnz_of_col``: entries of the plan's columns in their
+        order, most first."""
         goal = self.cfg.items_per_cta * self.grid
         fixed = self.cfg.segments > 0
-        if len(items) == 0 or (not fixed and len(items) >= goal):
+        ntiles, R = len(host_tiles), max(self.arena.R, 1)
+        if ntiles == 0 or (not fixed and ntiles * S >= goal):
             return None
-        windows = items[:, 5] - items[:, 4]
+        ncol = np.maximum(host_tiles[:, 3], 1)
+        windows = R / S
         # a part goes on past its own windows until each of its lanes has finished the FP32
         # run it is in: the windows in which the tile's sparsest column has one per lane
-        least = nnz_of_col[items[:, 2] + items[:, 3] - 1] / max(self.arena.R, 1)
-        tail = self.cfg.fold * -(-512 // np.maximum(items[:, 3], 1)) / np.maximum(least, 1e-9)
+        least = nnz_of_col[host_tiles[:, 2] + ncol - 1] / R
+        tail = self.cfg.fold * -(-512 // ncol) / np.maximum(least, 1e-9)
         if fixed:  # as the columns ask, so a pair's arithmetic does not depend on the rows
-            n = np.minimum(-(-windows // PART_WINDOWS), windows / np.maximum(4.0 * tail, 1.0))
+            n = np.minimum(math.ceil(windows / PART_WINDOWS), windows / np.maximum(4.0 * tail, 1.0))
             n = np.maximum(n, 1).astype(np.int64)
         else:
-            n = split_segments(windows, est, tail, self.grid, goal)
+            n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S, tail, S,
+                               self.grid, goal)
         if n.max() == 1:
             return None
-        order = np.argsort(items[:, 6], kind="stable")  # tiles in order, segments in order
-        first = np.empty(len(items), np.int64)
-        first[order] = np.cumsum(n[order]) - n[order]
-        of = np.repeat(np.arange(len(items)), n)        # item of each part, and its number
-        k = np.arange(len(of)) - np.repeat(np.cumsum(n) - n, n)
-        parts = np.zeros((len(of), 12), np.int64)
-        parts[:, 0:4] = items[of, 0:4]
-        parts[:, 4] = items[of, 4] + k * windows[of] // n[of]
-        parts[:, 5] = items[of, 4] + (k + 1) * windows[of] // n[of]
-        parts[:, 6] = first[of] + k
-        parts[:, 7] = items[of, 7]
-        parts[:, 8] = items[of, 4]
-        parts[:, 9] = items[of, 5]
-        tiles = np.zeros((len(host_tiles), 8), np.int64)
+        per_tile = n * S
+        tile = np.repeat(np.arange(ntiles), per_tile)
+        first = np.cumsum(per_tile) - per_tile
+        i = np.arange(len(tile)) - first[tile]  # part of the tile: segment i // n, part i % n
+        nt = n[tile]
+        s = i // nt
+        s0, s1 = s * R // S, (s + 1) * R // S
+        k, w = i - s * nt, s1 - s0
+        parts = np.zeros((len(tile), 12), np.int64)
+        parts[:, 0:4] = host_tiles[tile, 0:4]
+        parts[:, 4] = s0 + k * w // nt
+        parts[:, 5] = s0 + (k + 1) * w // nt
+        parts[:, 6] = np.arange(len(tile))
+        parts[:, 7] = tile
+        parts[:, 8] = s0
+        parts[:, 9] = s1
+        tiles = np.zeros((ntiles, 8), np.int64)
         tiles[:, 0:4] = host_tiles[:, 0:4]
-        tiles[:, 5] = np.bincount(items[:, 7], weights=n, minlength=len(host_tiles))
-        tiles[:, 4] = np.cumsum(tiles[:, 5]) - tiles[:, 5]
-        return parts[np.argsort(-(est / n)[of], kind="stable")], tiles
+        tiles[:, 4] = first
+        tiles[:, 5] = per_tile
+        return parts[np.argsort(-(cost / n)[tile], kind="stable")], tiles
 
     def plan_triangle(self, ids: Optional[Sequence[int]] = None, ldc: Optional[int] = None) -> PairPlan:
         """All pairs i < j among ``ids`` (default: every vector of the arena), and

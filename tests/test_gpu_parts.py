@@ -45,7 +45,7 @@ def test_parts_form_the_segments_sums(monkeypatch, alphabet, k, n, scale, cfg, p
     arena = _arena(alphabet, k, n, scale)
     # parts as short as `part` windows, also where their tails outweigh them
     monkeypatch.setattr(engine, "split_segments",
-                        lambda windows, *a: np.maximum(-(-windows // part), 1))
+                        lambda windows, *a: np.maximum(-(-windows // part), 1).astype(np.int64))
     monkeypatch.setattr(engine, "PART_WINDOWS", part)
     eng = PairEngine(arena, EngineConfig(**cfg))
     eng.ensure_index()
