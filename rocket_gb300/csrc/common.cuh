@@ -227,6 +227,34 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
 }
 
 // ------------------------------------------------------------------------
+// chains of short kernels
+// ------------------------------------------------------------------------
+
+// launch_next puts a kernel that starts with previous_kernel_done() behind the kernel
+// before it on the stream with its launch work already done when that one ends
+// (programmatic dependent launch; no kernel here signals early, so the next one's
+// blocks never take room from running ones).  A proteome of 30 proteins, ten kernels:
+// 121 -> 98 us for the call; signalling at the start of each kernel instead: 104.
+__device__ __forceinline__ void previous_kernel_done() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... K, typename... A>
+inline cudaError_t launch_next(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t st,
+                               A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// ------------------------------------------------------------------------
 // misc
 // ------------------------------------------------------------------------
 

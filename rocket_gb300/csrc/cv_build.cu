@@ -251,6 +251,7 @@ __device__ __forceinline__ uint32_t ext_mask(const BuildArgs &a, int p, uint32_t
 // sets tile_base[p] = number of TILE-sized tiles of proteomes < p (tile_base[B] =
 // total) and, for a single proteome, its offsets and output range.
 __global__ void __launch_bounds__(256) k_begin(BuildArgs a) {
+    previous_kernel_done();
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.zero_n8; i += step)
         a.zero[i] = 0;
@@ -326,6 +327,7 @@ __device__ __forceinline__ float div_by_scale(float f, double scale, double rs) 
 
 // Normalised value of every tuple, after the norm is known.  grid = (TUPLE_TABLE / 256, B)
 __global__ void k_tuple_value(BuildArgs a) {
+    previous_kernel_done();
     const int p = blockIdx.y;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (uint32_t)TUPLE_TABLE) return;
@@ -344,6 +346,7 @@ __global__ void k_tuple_value(BuildArgs a) {
 // alphabet and inside the proteome (native.cu:236-252).
 template <bool COMPACT>
 __global__ void __launch_bounds__(COUNT_THREADS) k_count(BuildArgs a) {
+    previous_kernel_done();
     __shared__ uint8_t dig[TILE + 16];
     __shared__ uint32_t ntot[3];
     const int K = a.k;
@@ -413,6 +416,9 @@ __global__ void __launch_bounds__(COUNT_THREADS) k_count(BuildArgs a) {
     }
 }
 
+// Consecutive bitmap words of a warp of the candidate passes.
+__device__ __forceinline__ uint32_t warp_words(const BuildArgs &a) { return a.wlanes * a.wpt; }
+
 // Candidates of the seen (K-1)-mers of one word of the seen bitmap (32
 // consecutive (K-1)-mers): |R(m)| = popc(ext_mask(m)) for each seen q = a.m.
 __device__ __forceinline__ uint32_t word_candidates(const BuildArgs &a, int p, uint32_t q0,
@@ -426,27 +432,35 @@ __device__ __forceinline__ uint32_t word_candidates(const BuildArgs &a, int p, u
     return s;
 }
 
-// Candidates and seen (K-1)-mers per chunk of CHUNK_THREADS * wpt bitmap words (wpt
-// consecutive words per thread: 8 for the sparse bitmaps of protein K = 7, else 1).
+// Candidates and seen (K-1)-mers per chunk of bitmap words: each of the CTA's warps has
+// warp_words(a) consecutive ones, wpt per lane (8 for the sparse bitmaps of protein K =
+// 7), or 32, 8 or 2 of them with 1, 4 or 16 lanes to a word (see chunk_words).
 // grid = (NCH + table blocks, B).  With compact (K-2)-mer tables also zeroes the entries
 // in use, which k_c0_scatter counts in.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
+    previous_kernel_done();
     const int p = blockIdx.y, c = blockIdx.x;
     if ((uint64_t)c >= a.NCH) {
         table_block(a, p, c - (int)a.NCH);
         return;
     }
     const uint64_t nw = a.T1s / 32;
-    const uint64_t wd0 = ((uint64_t)c * CHUNK_THREADS + threadIdx.x) * a.wpt;
+    const uint32_t lane = threadIdx.x & 31u, shared = 32u / a.wlanes;  // lanes to a word
+    const uint64_t wd0 = ((uint64_t)c * (CHUNK_THREADS / 32) + threadIdx.x / 32) * warp_words(a) +
+                         lane / shared * a.wpt;
     uint32_t s = 0, n = 0;
     for (uint32_t i = 0; i < a.wpt; i++) {
         const uint64_t wd = wd0 + i;
-        if (wd >= nw) break;
-        const uint32_t bits = a.seen1[(uint64_t)p * nw + wd];
-        const uint32_t sw = bits ? word_candidates(a, p, (uint32_t)(wd * 32), bits) : 0u;
-        a.word_cand[(uint64_t)p * nw + wd] = sw;
+        uint32_t bits = 0, sw = 0;
+        if (wd < nw) {
+            bits = a.seen1[(uint64_t)p * nw + wd];
+            if (shared > 1) bits &= ((1u << a.wlanes) - 1u) << (lane % shared * a.wlanes);
+            if (bits) sw = word_candidates(a, p, (uint32_t)(wd * 32), bits);
+        }
         s += sw;
         n += __popc(bits);
+        for (uint32_t d = 1; d < shared; d <<= 1) sw += __shfl_xor_sync(0xffffffffu, sw, d);
+        if (wd < nw && lane % shared == 0) a.word_cand[(uint64_t)p * nw + wd] = sw;
     }
     s = __reduce_add_sync(0xffffffffu, s);
     n = __reduce_add_sync(0xffffffffu, n);
@@ -479,6 +493,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
 // than the launches of a wider scan cost.
 constexpr int CSCAN_THREADS = 1024, CSCAN_ITEMS = 8;
 __global__ void __launch_bounds__(CSCAN_THREADS) k_cand_scan(BuildArgs a) {
+    previous_kernel_done();
     __shared__ uint64_t sw[CSCAN_THREADS / 32 + 1];
     const uint64_t nc = (uint64_t)a.B * a.NCH;
     uint64_t cand = 0, seen = 0;  // before the round
@@ -559,13 +574,12 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t i) {
 
 // coff[p][q] = candidate offset of seen (K-1)-mer q within proteome p (entries
 // of unseen q are not written); cq = the key q * A + b of every candidate (b over
-// the right-extension mask of q's suffix, ascending), c0a zeroed.  Thread t of
-// the block owns bitmap words [(c * CHUNK_THREADS + t) * wpt, + wpt) and its
-// candidates and seen (K-1)-mers start at the exclusive scans of the word_cand sums and
+// the right-extension mask of q's suffix, ascending), c0a zeroed.  A warp owns a
+// contiguous run of bitmap words, wpt per lane of its first wlanes, and their candidates;
+// these and the seen (K-1)-mers start at the exclusive scans of the word_cand sums and
 // the words' populations (one scan of packed pairs; with compact tables pw1 gets the
-// ranks of the words that hold any); a warp's 32
-// threads own a contiguous run of words and candidates, which the warp
-// processes together: its seen (K-1)-mers, 32 at a time in order (each lane
+// ranks of the words that hold any).  The warp
+// processes its run together: its seen (K-1)-mers, 32 at a time in order (each lane
 // finds its own by a search over the scan of the words' populations), load
 // their masks together; a warp scan of the mask populations places their
 // candidates, each lane writes its candidates into the warp's shared-memory stage
@@ -576,6 +590,7 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t i) {
 // scan cost about three times the instructions of the stage.)
 // grid = (NCH, B)
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
+    previous_kernel_done();
     __shared__ uint64_t sw[CHUNK_THREADS / 32 + 1];
     __shared__ uint32_t s_stage[CHUNK_THREADS / 32][32 * 21];  // keys of 32 seen (K-1)-mers (A <= 21)
     uint32_t *stage = s_stage[threadIdx.x >> 5];
@@ -584,9 +599,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
     const uint64_t pc = (uint64_t)p * a.NCH + c;
     const uint64_t nw = a.T1s / 32;
     const uint32_t *seen = a.seen1 + (uint64_t)p * nw;
-    const uint64_t wd0 = ((uint64_t)c * CHUNK_THREADS + threadIdx.x) * a.wpt;
+    const uint64_t wbeg =
+        ((uint64_t)c * (CHUNK_THREADS / 32) + threadIdx.x / 32) * warp_words(a);
+    const uint64_t wd0 = wbeg + lane * a.wpt;
     uint32_t s = 0, npop = 0;
-    for (uint32_t i = 0; i < a.wpt && wd0 + i < nw; i++) {
+    for (uint32_t i = 0; i < a.wpt && lane < a.wlanes && wd0 + i < nw; i++) {
         s += a.word_cand[(uint64_t)p * nw + wd0 + i];
         npop += __popc(seen[wd0 + i]);
     }
@@ -603,8 +620,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
     for (uint64_t i = gb + run + lane; i < gb + r1 && i < a.cand_cap; i += 32) a.c0a[i] = 0u;
     // the warp's words [wbeg, wend), loaded up front (coalesced), lane l holding word
     // wbeg + 32 t + l of group t; the seen (K-1)-mers of a group are taken 32 at a time
-    const uint64_t wbeg = __shfl_sync(0xffffffffu, wd0, 0);
-    const uint64_t wend = min(wbeg + (uint64_t)32 * a.wpt, nw);
+    const uint64_t wend = min(wbeg + warp_words(a), nw);
     const uint32_t A = a.A;
     uint32_t wreg[MAX_WPT];
 #pragma unroll
@@ -622,7 +638,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
         const uint64_t wfirst = wbeg + 32 * t;
         // compact tables: P is the rank of the group's first seen (K-1)-mer; the i-th seen
         // (K-1)-mer of the group is then entry P + i
-        if (a.compact1 && wfirst + lane < nw)
+        if (a.compact1 && wfirst + lane < wend)
             a.pw1[(uint64_t)p * nw + wfirst + lane] = make_uint2(P + wincl - __popc(wbits), wbits);
         for (uint32_t sb = 0; sb < nseen; sb += 32) {
             const uint32_t i = sb + lane;
@@ -677,6 +693,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
 // instead of two measured no faster, and one 64-bit atomic for count and offset instead
 // of an atomic and a load took the build of 200 uneven proteomes from 22.2 to 21.0 ms.
 __global__ void __launch_bounds__(COUNT_THREADS) k_c0_scatter(BuildArgs a) {
+    previous_kernel_done();
     __shared__ uint8_t dig[TILE + 16];
     const int K = a.k;
     const uint32_t A = a.A;
@@ -775,6 +792,7 @@ constexpr int ALPHA_ILP = 1;  // listed candidates per lane in flight together
 // 0x7fffffff) has these bits.
 constexpr uint32_t CAND_DROP = 0xffffffffu;
 __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
+    previous_kernel_done();
     __shared__ U192 s_norm[CHUNK_THREADS / 32];
     __shared__ uint32_t s_m1[CHUNK_THREADS / 32], s_bad[CHUNK_THREADS / 32],
         s_surv[CHUNK_THREADS / 32];
@@ -908,6 +926,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
 // summed exactly, in any order).
 constexpr int NORM_THREADS = 512, NORM_ITEMS = 4;
 __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
+    previous_kernel_done();
     __shared__ U192 s_acc[NORM_THREADS / 32];
     __shared__ uint64_t s_m1[NORM_THREADS / 32], sw[NORM_THREADS / 32 + 1];
     __shared__ uint32_t s_bad[NORM_THREADS / 32];
@@ -983,11 +1002,12 @@ __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
 // one or two atomics per seen (K-1)-mer instead of one per written key.  The
 // marked set is a superset of the written keys (a candidate whose alpha is 0 is
 // marked but not written), which is all a key-rank bitmap needs: ranks stay
-// strictly increasing over the written keys.  grid = (NCH, B)
+// strictly increasing over the written keys.  grid = (words / (CHUNK_THREADS * wpt), B)
 __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
-    const int p = blockIdx.y, c = blockIdx.x;
+    previous_kernel_done();
+    const int p = blockIdx.y;
     const uint64_t nw = a.T1s / 32;
-    const uint64_t wd0 = ((uint64_t)c * CHUNK_THREADS + threadIdx.x) * a.wpt;
+    const uint64_t wd0 = ((uint64_t)blockIdx.x * CHUNK_THREADS + threadIdx.x) * a.wpt;
     for (uint32_t i = 0; i < a.wpt; i++) {
         const uint64_t wd = wd0 + i;
         if (wd >= nw) break;
@@ -1018,6 +1038,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
 // a.pad_blocks more, which fill the rest of its output with the padding of
 // native.cu:473-474; a single proteome that does not fit leaves its output as it is.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_compact(BuildArgs a) {
+    previous_kernel_done();
     __shared__ uint64_t s_base[SMEM_BASES + 1];
     if (a.single && (*a.status || a.nnz[0] > a.single_cap)) return;
     const uint64_t c = blockIdx.x, g0 = c * ALPHA_TILE, ncta = a.cand_cap / ALPHA_TILE;
@@ -1122,8 +1143,24 @@ int build_geometry(int alpha, int k, BuildGeometry *g) {
     g->T2 = ipow64(A, k - 2);
     g->T2s = (g->T2 + 31) / 32 * 32;
     g->wpt = g->T1s > (1ull << 24) ? MAX_WPT : 1;  // sparse bitmaps: eight words per thread
-    g->NCH = div_up(g->T1s / 32, (uint64_t)CHUNK_THREADS * g->wpt);
     return 0;
+}
+
+// Lanes with words per warp of the candidate passes for B proteomes: 32, or 8 or 2 where
+// that leaves fewer than MIN_CHUNKS CTAs.  A word's (K-1)-mers share all but their last
+// symbols, so its work goes with the frequencies of those symbols, and with few CTAs
+// the densest words are what the pass waits for (one proteome of 1,500 proteins at K = 6,
+// 499 CTAs: k_cand_offsets 30 us at 22% of the warp slots; with 1,995 the whole call
+// 141 -> 135 us; 3,000 proteins at K = 5, 24 -> 380 CTAs: 234 -> 180 us).  Proteomes of
+// few residues have no such words, and at K = 6 the extra CTAs cost more than they give
+// (30 proteins: 97 -> 112 us): build_plan keeps 32 there.
+constexpr uint64_t MIN_CHUNKS = 1500, SHORT_PROTEOME = 1u << 18;
+static uint32_t chunk_lanes(const BuildGeometry &g, int B) {
+    uint32_t lanes = 32;
+    if (g.wpt == 1)
+        while (lanes > 2 && (uint64_t)B * div_up(g.T1s / 32, CHUNK_THREADS / 32 * lanes) < MIN_CHUNKS)
+            lanes /= 4;
+    return lanes;
 }
 
 // (K-1)-mer tables beyond 2^20 entries per proteome (protein K >= 6) are kept
@@ -1144,13 +1181,15 @@ static uint64_t cand_cap_rounded(uint64_t cand_cap) {
 // with every array in order.
 template <typename Take>
 static void build_layout(const BuildGeometry &g, int B, uint64_t cand_cap, BuildArgs &r, Take &&take) {
-    const uint64_t nc = (uint64_t)B * g.NCH;
+    r.wpt = g.wpt;
+    r.wlanes = chunk_lanes(g, B);
+    r.NCH = div_up(g.T1s / 32, (uint64_t)(CHUNK_THREADS / 32) * r.wlanes * r.wpt);
+    const uint64_t nc = (uint64_t)B * r.NCH;
     const uint64_t cap = cand_cap_rounded(cand_cap);
     const uint64_t ncta = cap / ALPHA_TILE, nseg = cap / SEG;
     const uint64_t nw1 = g.T1s / 32 * B, nw2 = g.T2s / 32 * B;
     const bool compact = compact1_tables(g), compact2 = compact2_tables(g);
-    r.alpha = g.alpha; r.k = g.k; r.A = g.A; r.T1 = g.T1; r.T2 = g.T2; r.NCH = g.NCH; r.B = B;
-    r.wpt = g.wpt;
+    r.alpha = g.alpha; r.k = g.k; r.A = g.A; r.T1 = g.T1; r.T2 = g.T2; r.B = B;
     r.T1s = g.T1s;
     r.T2s = g.T2s;
     r.fdT2.set((uint32_t)g.T2);
@@ -1227,23 +1266,30 @@ cudaError_t build_carve(const BuildGeometry &g, int B, uint64_t cand_cap, void *
 
 // Phase 1: everything up to per-proteome nnz (no host sync inside).
 cudaError_t build_plan(BuildArgs &a, cudaStream_t st) {
+    if (a.single && a.compact1 && a.wpt == 1 && a.single_len < SHORT_PROTEOME) {
+        a.wlanes = 32;
+        a.NCH = div_up(a.T1s / 32, (uint64_t)CHUNK_THREADS);
+    }
     const int sms = device_sm_count();
     const uint64_t zero_blocks = div_up(a.zero_n8, 4 * 256);
-    k_begin<<<(unsigned)max((uint64_t)1, min(zero_blocks, (uint64_t)sms * 8)), 256, 0, st>>>(a);
+    const unsigned B = (unsigned)a.B, nch = (unsigned)a.NCH;
+    PHYLO_CHECK(launch_next(k_begin,
+                            (unsigned)max((uint64_t)1, min(zero_blocks, (uint64_t)sms * 8)), 256,
+                            st, a));
     const int grid_seq = sms * 8;
-    if (a.compact1) k_count<true><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
-    else k_count<false><<<grid_seq, COUNT_THREADS, 0, st>>>(a);
+    PHYLO_CHECK(launch_next(a.compact1 ? k_count<true> : k_count<false>, grid_seq, COUNT_THREADS,
+                            st, a));
     if (a.compact2)  // ranks of the seen (K-2)-mers
         PHYLO_CHECK(bitmap_prefix_pairs(a.seen2, a.T2s / 32 * a.B, a.p2_partials, a.pw2,
                                         a.p2_total, st));
-    k_cand_count<<<dim3((unsigned)a.NCH + PROB_BLOCKS + TUPLE_BLOCKS, (unsigned)a.B), CHUNK_THREADS,
-                   0, st>>>(a);
-    k_cand_scan<<<1, CSCAN_THREADS, 0, st>>>(a);
-    k_cand_offsets<<<dim3((unsigned)a.NCH, (unsigned)a.B), CHUNK_THREADS, 0, st>>>(a);
-    k_c0_scatter<<<grid_seq, COUNT_THREADS, 0, st>>>(a);
-    k_alpha<<<(unsigned)(a.cand_cap / ALPHA_TILE), CHUNK_THREADS, 0, st>>>(a);
-    k_norm<<<a.B, NORM_THREADS, 0, st>>>(a);
-    k_tuple_value<<<dim3(TUPLE_TABLE / 256, a.B), 256, 0, st>>>(a);
+    PHYLO_CHECK(launch_next(k_cand_count, dim3(nch + PROB_BLOCKS + TUPLE_BLOCKS, B), CHUNK_THREADS,
+                            st, a));
+    PHYLO_CHECK(launch_next(k_cand_scan, 1, CSCAN_THREADS, st, a));
+    PHYLO_CHECK(launch_next(k_cand_offsets, dim3(nch, B), CHUNK_THREADS, st, a));
+    PHYLO_CHECK(launch_next(k_c0_scatter, grid_seq, COUNT_THREADS, st, a));
+    PHYLO_CHECK(launch_next(k_alpha, (unsigned)(a.cand_cap / ALPHA_TILE), CHUNK_THREADS, st, a));
+    PHYLO_CHECK(launch_next(k_norm, B, NORM_THREADS, st, a));
+    PHYLO_CHECK(launch_next(k_tuple_value, dim3(TUPLE_TABLE / 256, B), 256, st, a));
     return cudaGetLastError();
 }
 
@@ -1253,9 +1299,12 @@ cudaError_t build_emit(BuildArgs &a, cudaStream_t st) {
     if (a.single)
         a.pad_blocks = (unsigned)min(div_up(a.single_cap ? a.single_cap : 1, 8 * CHUNK_THREADS),
                                      (uint64_t)device_sm_count() * 8);
-    k_compact<<<(unsigned)(ncta + a.pad_blocks), CHUNK_THREADS, 0, st>>>(a);
+    PHYLO_CHECK(launch_next(k_compact, (unsigned)(ncta + a.pad_blocks), CHUNK_THREADS, st, a));
     if (a.union_bits)
-        k_union_mark<<<dim3((unsigned)a.NCH, (unsigned)a.B), CHUNK_THREADS, 0, st>>>(a);
+        PHYLO_CHECK(launch_next(k_union_mark,
+                                dim3((unsigned)div_up(a.T1s / 32, (uint64_t)CHUNK_THREADS * a.wpt),
+                                     (unsigned)a.B),
+                                CHUNK_THREADS, st, a));
     return cudaGetLastError();
 }
 

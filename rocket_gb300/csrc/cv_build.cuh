@@ -10,7 +10,6 @@ struct BuildGeometry {
     uint64_t T1, T2; // A^(K-1), A^(K-2)
     uint64_t T1s;    // per-proteome row length of the (K-1)-mer tables (T1 rounded up to 32)
     uint64_t T2s;    // the same for the (K-2)-mer tables
-    uint64_t NCH;    // chunks of the seen bitmap per proteome (CHUNK_THREADS * wpt words)
     uint32_t wpt;    // bitmap words per thread in the candidate passes
 };
 
@@ -51,8 +50,9 @@ constexpr uint32_t TUPLE_TAG = 0xffff0000u;
 struct BuildArgs {
     int alpha, k, B;
     uint32_t A;
-    uint64_t T1, T2, T1s, T2s, NCH;
-    uint32_t wpt;
+    uint64_t T1, T2, T1s, T2s;
+    uint64_t NCH;             // chunks of the seen bitmap per proteome (one CTA's words)
+    uint32_t wpt, wlanes;     // bitmap words per lane, and lanes with words per warp
     // input: concatenated sequences, seq_off[B+1] (device)
     const uint8_t *seq;
     const uint64_t *seq_off;
