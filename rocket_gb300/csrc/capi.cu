@@ -25,6 +25,7 @@
 #include "allpairs.cuh"
 #include "compare.cuh"
 #include "cv_build.cuh"
+#include "hostctx.cuh"
 #include "postings.cuh"
 #include "rank.cuh"
 #include "scan.cuh"
@@ -151,16 +152,19 @@ int buildCompositionVector(uintptr_t stream, uintptr_t d_temp_storage_ptr, long 
     a.single = 1;
     a.single_len = (uint64_t)string_len;
     a.single_cap = max_size;
-    PHYLO_CHECK(build_plan(a, st));
-    PHYLO_CHECK(build_emit(a, st));  // writes nothing where the checks below fail
-    // one read-back for the whole call: nnz | norm | candidates | status
-    struct {
-        uint64_t nnz;
-        double norm;
-        uint64_t candidates;
-        uint32_t status;
-    } res;
-    PHYLO_CHECK(cudaMemcpyAsync(&res, a.nnz, 28, cudaMemcpyDeviceToHost, st));
+    // the whole call's results: nnz, norm, candidates and status, in the order they have
+    // in scratch; k_norm leaves them here where the device can write host memory
+    SingleResult res = {};
+    const bool direct = device_uses_host_memory();
+    a.host_result = direct ? &res : nullptr;
+    err = build_plan(a, st);
+    if (err == cudaSuccess) err = build_emit(a, st);  // writes nothing where the checks below fail
+    if (err != cudaSuccess) {
+        cudaStreamSynchronize(st);  // what was queued may still write to res
+        return (int)err;
+    }
+    if (!direct)
+        PHYLO_CHECK(cudaMemcpyAsync(&res, a.nnz, sizeof(res), cudaMemcpyDeviceToHost, st));
     PHYLO_CHECK(cudaStreamSynchronize(st));
     if (h_size) *h_size = (uint32_t)res.nnz;
     if (res.status & DEV_CAPACITY) {
@@ -180,6 +184,28 @@ int buildCompositionVector(uintptr_t stream, uintptr_t d_temp_storage_ptr, long 
     return (int)cudaGetLastError();
 }
 
+// A pair compare and its status: `launch` queues the kernels, with the address they
+// leave the status in (a host variable where the device can write it, else null).
+}  // extern "C"
+
+template <typename Launch>
+static int compare_and_wait(cudaStream_t st, Launch launch) {
+    uint32_t *d_status = nullptr;
+    uint32_t status = DEV_WAIT_TIMEOUT;
+    const bool direct = device_uses_host_memory();
+    const cudaError_t e = launch(&d_status, direct ? &status : nullptr);
+    if (e != cudaSuccess) return (int)e;
+    if (direct) PHYLO_CHECK(cudaStreamSynchronize(st));
+    else PHYLO_CHECK(last_status(d_status, st, &status));
+    if (status) {
+        fprintf(stderr, "error: compare kernel reported device status %u\n", status);
+        return (int)cudaErrorLaunchTimeout;
+    }
+    return (int)cudaGetLastError();
+}
+
+extern "C" {
+
 int compareCompositionVectors(uintptr_t stream, uintptr_t d_temp_storage_ptr, long temp_storage_size,
                               uintptr_t d_left_keys_ptr, uintptr_t d_left_values_ptr, int left_size,
                               uintptr_t d_right_keys_ptr, uintptr_t d_right_values_ptr,
@@ -190,19 +216,15 @@ int compareCompositionVectors(uintptr_t stream, uintptr_t d_temp_storage_ptr, lo
         return (int)cudaErrorInvalidValue;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t *d_status = nullptr;
-    PHYLO_CHECK(compare_launch(st, (void *)d_temp_storage_ptr, (size_t)temp_storage_size,
-                               (const uint32_t *)d_left_keys_ptr, (const float *)d_left_values_ptr,
-                               (uint32_t)left_size, (const uint32_t *)d_right_keys_ptr,
-                               (const float *)d_right_values_ptr, (uint32_t)right_size,
-                               (double *)d_output_ptr, &d_status));
-    uint32_t status = 0;
-    PHYLO_CHECK(last_status(d_status, st, &status));
-    if (status) {
-        fprintf(stderr, "error: compare kernel reported device status %u\n", status);
-        return (int)cudaErrorLaunchTimeout;
-    }
-    return (int)cudaGetLastError();
+    return compare_and_wait(st, [&](uint32_t **d_status, uint32_t *host_status) -> cudaError_t {
+        PHYLO_CHECK(compare_launch(st, (void *)d_temp_storage_ptr, (size_t)temp_storage_size,
+                                   (const uint32_t *)d_left_keys_ptr,
+                                   (const float *)d_left_values_ptr, (uint32_t)left_size,
+                                   (const uint32_t *)d_right_keys_ptr,
+                                   (const float *)d_right_values_ptr, (uint32_t)right_size,
+                                   (double *)d_output_ptr, d_status, host_status));
+        return cudaSuccess;
+    });
 }
 
 // For callers that cannot allocate device memory (see include/phylogenetics.h):
@@ -217,19 +239,13 @@ int compareCompositionVectorsStatic(uintptr_t stream, uintptr_t d_left_keys_ptr,
         return (int)cudaErrorInvalidValue;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t *d_status = nullptr;
-    cudaError_t e = compare_launch_static(
-        st, (const uint32_t *)d_left_keys_ptr, (const float *)d_left_values_ptr,
-        (uint32_t)left_size, (const uint32_t *)d_right_keys_ptr,
-        (const float *)d_right_values_ptr, (uint32_t)right_size, (double *)d_output_ptr, &d_status);
-    if (e != cudaSuccess) return (int)e;
-    uint32_t status = 0;
-    PHYLO_CHECK(last_status(d_status, st, &status));
-    if (status) {
-        fprintf(stderr, "error: compare kernel reported device status %u\n", status);
-        return (int)cudaErrorLaunchTimeout;
-    }
-    return (int)cudaGetLastError();
+    return compare_and_wait(st, [&](uint32_t **d_status, uint32_t *host_status) {
+        return compare_launch_static(st, (const uint32_t *)d_left_keys_ptr,
+                                     (const float *)d_left_values_ptr, (uint32_t)left_size,
+                                     (const uint32_t *)d_right_keys_ptr,
+                                     (const float *)d_right_values_ptr, (uint32_t)right_size,
+                                     (double *)d_output_ptr, d_status, host_status);
+    });
 }
 
 int phyloCompareTileElements(void) { return (int)compare_tile_elements(); }

@@ -21,8 +21,8 @@
 // the answer (the ones the tile's copies read) rather than sectors scattered
 // over both lists.
 //
-// k_compare (one pair, one launch) keeps a running sum per thread and combines
-// the CTAs' partials in a fixed order in the last CTA; k_many_intersect (many
+// k_compare (one pair) keeps a running sum per thread and leaves one partial per CTA,
+// which k_compare_sum combines in a fixed order; k_many_intersect (many
 // pairs, tiles of all pairs in one index space) leaves one partial per tile,
 // which k_many_reduce sums per pair in tile order.  Every wait is bounded; a
 // timed-out wait records DEV_WAIT_TIMEOUT, the producer stops issuing and waits
@@ -49,12 +49,10 @@ constexpr uint32_t CMP_MIN_CAP = 1024;  // partial slots always carved
 constexpr uint32_t CMP_WAIT = 1u << 22; // default poll limit of a wait
 constexpr uint32_t CMP_DRAIN = 1u << 16;
 
-// Completion ticket and status first (cleared before every launch), then one
-// float-float partial per CTA.
+// The status, then one float-float partial per CTA; every word is written by the
+// kernels of a call before it is read, so nothing needs clearing.
 struct CmpState {
-    uint32_t ticket;
-    uint32_t status;
-    uint32_t pad[2];
+    uint32_t unused0, status, unused1[2];
     FF partial[1];  // [cmp_partials(ntiles)]
 };
 
@@ -374,15 +372,24 @@ __device__ __forceinline__ void pipe_init(Pipe &pp) {
     __syncthreads();
 }
 
+// The partial of a CTA whose wait ran out: NaN patterns that no arithmetic yields (its
+// NaNs are 0x7fffffff).
+__device__ __forceinline__ FF timed_out() {
+    return FF{__uint_as_float(0xffffdeadu), __uint_as_float(0xffffbeefu)};
+}
+__device__ __forceinline__ bool is_timed_out(FF p) {
+    return __float_as_uint(p.hi) == 0xffffdeadu && __float_as_uint(p.lo) == 0xffffbeefu;
+}
+
 __global__ void __launch_bounds__(CMP_THREADS) k_compare(
     const uint32_t *__restrict__ Ak, const float *__restrict__ Av, uint32_t na,
     const uint32_t *__restrict__ Bk, const float *__restrict__ Bv, uint32_t nb, uint32_t ntiles,
-    uint32_t per, uint32_t first_wait_limit, CmpState *st, double *out) {
+    uint32_t per, uint32_t first_wait_limit, FF *partial) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ Pipe pp;
-    __shared__ uint32_t s_split[CMP_MAX_RUN + 1];
+    __shared__ uint32_t s_split[CMP_MAX_RUN + 1], s_status;
     __shared__ FF s_final[CMP_CONSUMERS];
-    __shared__ bool s_last;
+    if (threadIdx.x == 0) s_status = DEV_OK;
     const uint64_t total = (uint64_t)na + nb;
     const uint64_t t_begin = (uint64_t)blockIdx.x * per;
     const uint64_t t_end = min((uint64_t)ntiles, t_begin + per);
@@ -396,42 +403,47 @@ __global__ void __launch_bounds__(CMP_THREADS) k_compare(
     pipe_init(pp);  // (its barrier also publishes the splits)
     if (threadIdx.x >= CMP_CONSUMER_THREADS) {
         if (t_begin < t_end)
-            produce_one(Ak, Av, na, Bk, Bv, nb, s_split, t_begin, t_end, pp, smem_raw,
-                        &st->status);
+            produce_one(Ak, Av, na, Bk, Bv, nb, s_split, t_begin, t_end, pp, smem_raw, &s_status);
         return;
     }
     FF acc = {0.0f, 0.0f};
-    consume<false>(t_begin, t_end, pp, smem_raw, first_wait_limit, nullptr, acc, &st->status);
-    // CTA reduction (consumer warps), then the last CTA combines in a fixed order
+    consume<false>(t_begin, t_end, pp, smem_raw, first_wait_limit, nullptr, acc, &s_status);
+    // CTA reduction (consumer warps); a CTA that gave up leaves TIMED_OUT
     acc = ff_warp_sum(acc);
     if ((threadIdx.x & 31) == 0) s_final[threadIdx.x >> 5] = acc;
     consumers_sync();
     if (threadIdx.x == 0) {
         FF r = {0.0f, 0.0f};
         for (int w = 0; w < CMP_CONSUMERS; w++) r = ff_merge(r, s_final[w]);
-        st->partial[blockIdx.x] = r;
-        __threadfence();
-        const uint32_t done = atomicAdd(&st->ticket, 1u);
-        s_last = (done == gridDim.x - 1);
+        partial[blockIdx.x] = *(volatile uint32_t *)&s_status ? timed_out() : r;
     }
-    consumers_sync();
-    if (s_last && threadIdx.x < 32) {
-        __threadfence();
-        // lane l sums partials l, l+32, ... in double-double, then a fixed tree
-        DD dacc = {0.0, 0.0};
-        for (uint32_t c = threadIdx.x; c < gridDim.x; c += 32) {
-            const volatile float *p = reinterpret_cast<volatile float *>(&st->partial[c]);
-            dd_add(dacc, (double)p[0]);
-            dd_add(dacc, (double)p[1]);
-        }
+}
+
+// One warp: lane l sums partials l, l + 32, ... in double-double, then a fixed tree.  The
+// status also goes to *host_status, unless null.
+__global__ void __launch_bounds__(32) k_compare_sum(uint32_t n, CmpState *st, double *out,
+                                                    uint32_t *host_status) {
+    previous_kernel_done();
+    DD dacc = {0.0, 0.0};
+    bool bad = false;
+    for (uint32_t c = threadIdx.x; c < n; c += 32) {
+        const FF p = st->partial[c];
+        bad |= is_timed_out(p);
+        dd_add(dacc, (double)p.hi);
+        dd_add(dacc, (double)p.lo);
+    }
 #pragma unroll
-        for (int dd = 16; dd > 0; dd >>= 1) {
-            DD o;
-            o.hi = __shfl_down_sync(0xffffffffu, dacc.hi, dd);
-            o.lo = __shfl_down_sync(0xffffffffu, dacc.lo, dd);
-            dacc = dd_merge(dacc, o);
-        }
-        if (threadIdx.x == 0) *out = __dadd_rn(dacc.hi, dacc.lo);
+    for (int dd = 16; dd > 0; dd >>= 1) {
+        DD o;
+        o.hi = __shfl_down_sync(0xffffffffu, dacc.hi, dd);
+        o.lo = __shfl_down_sync(0xffffffffu, dacc.lo, dd);
+        dacc = dd_merge(dacc, o);
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (threadIdx.x == 0) {
+        st->status = bad ? DEV_WAIT_TIMEOUT : DEV_OK;
+        if (host_status) *host_status = bad ? DEV_WAIT_TIMEOUT : DEV_OK;
+        *out = __dadd_rn(dacc.hi, dacc.lo);
     }
 }
 
@@ -462,7 +474,8 @@ static cudaError_t compare_attributes() {
 
 cudaError_t compare_launch(cudaStream_t stream, void *scratch, size_t scratch_size,
                            const uint32_t *lk, const float *lv, uint32_t nl, const uint32_t *rk,
-                           const float *rv, uint32_t nr, double *d_out, uint32_t **status_out) {
+                           const float *rv, uint32_t nr, double *d_out, uint32_t **status_out,
+                           uint32_t *host_status) {
     const uint64_t total = (uint64_t)nl + nr;
     const uint32_t ntiles = (uint32_t)div_up(total, CMP_TILE);
     if (scratch_size < cmp_state_bytes(total) || scratch == nullptr) {
@@ -474,11 +487,8 @@ cudaError_t compare_launch(cudaStream_t stream, void *scratch, size_t scratch_si
     }
     CmpState *st = (CmpState *)scratch;
     if (status_out) *status_out = &st->status;
-    PHYLO_CHECK(cudaMemsetAsync(st, 0, 16, stream));  // ticket and status
-    if (ntiles == 0) {
-        // empty: C = 0
-        PHYLO_CHECK(cudaMemsetAsync(d_out, 0, sizeof(double), stream));
-        return cudaSuccess;
+    if (ntiles == 0) {  // empty: C = 0
+        return launch_next(k_compare_sum, 1, 32, stream, 0u, st, d_out, host_status);
     }
     PHYLO_CHECK(compare_attributes());
     // two CTAs per SM (three fit): one pair's split searches and the last CTA's
@@ -490,7 +500,8 @@ cudaError_t compare_launch(cudaStream_t stream, void *scratch, size_t scratch_si
     if (per > CMP_MAX_RUN) per = CMP_MAX_RUN;
     grid = (uint32_t)div_up(ntiles, per);
     k_compare<<<grid, CMP_THREADS, kCmpSmem, stream>>>(lk, lv, nl, rk, rv, nr, ntiles, per,
-                                                       g_first_wait_limit.load(), st, d_out);
+                                                       g_first_wait_limit.load(), st->partial);
+    PHYLO_CHECK(launch_next(k_compare_sum, 1, 32, stream, grid, st, d_out, host_status));
     return cudaGetLastError();
 }
 
@@ -509,8 +520,7 @@ cudaError_t compare_launch(cudaStream_t stream, void *scratch, size_t scratch_si
 // Limit: the two vectors may hold at most kStaticCompareMaxEntries entries
 // together (2^26 = 67,108,864), which needs kStaticCompareBytes of scratch.
 // All calls share the one array and it keeps what the last call left in it;
-// the partition kernel clears the completion ticket and the status word at the
-// start of every call, and every other byte a call reads it wrote first.  Two
+// every byte a call reads it wrote first.  Two
 // calls whose kernels overlap on the GPU (different streams, or different host
 // threads) would race on the array, so such calls must be serialised.
 // ---------------------------------------------------------------------------
@@ -546,7 +556,8 @@ static cudaError_t static_scratch_address(void **ptr) {
 
 cudaError_t compare_launch_static(cudaStream_t stream, const uint32_t *lk, const float *lv,
                                   uint32_t nl, const uint32_t *rk, const float *rv, uint32_t nr,
-                                  double *d_out, uint32_t **status_out) {
+                                  double *d_out, uint32_t **status_out,
+                                  uint32_t *host_status) {
     if ((uint64_t)nl + nr > kStaticCompareMaxEntries) {
         fprintf(stderr,
                 "error: vectors of %u and %u entries exceed the %llu entries the built-in scratch "
@@ -558,7 +569,7 @@ cudaError_t compare_launch_static(cudaStream_t stream, const uint32_t *lk, const
     void *scratch = nullptr;
     PHYLO_CHECK(static_scratch_address(&scratch));
     return compare_launch(stream, scratch, kStaticCompareBytes, lk, lv, nl, rk, rv, nr, d_out,
-                          status_out);
+                          status_out, host_status);
 }
 
 // ---------------------------------------------------------------------------

@@ -994,6 +994,7 @@ __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
         a.scale[p] = scale;
         a.rscale[p] = __ddiv_rn(1.0, scale);
         a.nnz[p] = run;
+        if (a.host_result) *a.host_result = {run, norm, *a.cand_total, *a.status, 0u};
     }
 }
 

@@ -46,6 +46,15 @@ constexpr int TUPLE_TABLE = TUPLE_FULL * TUPLE_PS * TUPLE_PS * TUPLE_MID;  // 32
 // place of its alpha bits (a negative-NaN pattern no computed alpha produces).
 constexpr uint32_t TUPLE_TAG = 0xffff0000u;
 
+// Results of a single proteome's build, in the order they have in scratch (nnz, norm,
+// cand_total, status).
+struct SingleResult {
+    uint64_t nnz;
+    double norm;
+    uint64_t candidates;
+    uint32_t status, unused;
+};
+
 // Everything a build launch needs; plain device pointers, passed by value.
 struct BuildArgs {
     int alpha, k, B;
@@ -114,6 +123,7 @@ struct BuildArgs {
     int single;
     uint64_t single_len, single_cap;
     unsigned pad_blocks;
+    SingleResult *host_result;  // where k_norm leaves them too, or null
     // K-mer counts per candidate, replaced by alpha bits
     uint32_t *c0a;
     uint64_t cand_cap;

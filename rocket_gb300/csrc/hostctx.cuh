@@ -107,4 +107,24 @@ inline int device_sm_count() {
     return n;
 }
 
+// Whether the current device reads and writes ordinary host memory through the host's
+// page tables (GB300 beside its Grace CPU), cached per device number.  A synchronous
+// call's kernel then leaves its few bytes of results in the caller's own variable,
+// instead of a read-back copy of 10 us behind it.
+inline bool device_uses_host_memory() {
+    static std::atomic<int> known[64];  // 0 not asked, 1 no, 2 yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        int v = 0;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) !=
+            cudaSuccess)
+            v = 0;
+        k = v ? 2 : 1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
+}
+
 }  // namespace phylo
