@@ -9,9 +9,9 @@
 //
 //   * one producer warp issues 1-D bulk copies (TMA) of each tile's left and
 //     right key/value ranges into a ring of two shared-memory stages, each
-//     completed on an mbarrier; the tiles' splits are known before it starts
-//     (one pair: the CTA's warps find its few boundaries together; many pairs:
-//     a kernel finds every boundary, a thread each);
+//     completed on an mbarrier (one pair: it finds the end of a tile from its start
+//     while earlier copies are in flight; many pairs: a kernel finds every boundary
+//     first, a thread each);
 //   * eight consumer warps merge a staged tile: a per-thread merge path over 17
 //     diagonals, products split exactly (TwoProduct) and summed as float-float
 //     (TwoSum); each warp releases the stage on the stage's "empty" mbarrier.
@@ -69,16 +69,17 @@ __host__ __device__ constexpr size_t cmp_state_bytes(uint64_t max_total) {
 size_t compare_scratch_bytes(uint64_t max_total) { return cmp_state_bytes(max_total); }
 
 // i = number of left elements before merged position d (ties to the left list),
-// found by a warp.  The predicate "A[i-1] <= B[d-i]" holds for i up to the split
-// and fails above it.  With step > 0 the first round probes 32 positions
-// `step` apart around `guess`; when the split lies among them the remaining
+// found by a warp, known to lie in [from, to].  The predicate "A[i-1] <= B[d-i]" holds
+// for i up to the split and fails above it.  With step > 0 the first round probes 32
+// positions `step` apart around `guess`; when the split lies among them the remaining
 // rounds stay inside one step.
 __device__ __forceinline__ uint32_t warp_merge_path(uint64_t d, const uint32_t *__restrict__ A,
                                                     uint32_t na, const uint32_t *__restrict__ B,
-                                                    uint32_t nb, uint64_t guess, uint32_t step) {
+                                                    uint32_t nb, uint32_t from, uint32_t to,
+                                                    uint64_t guess, uint32_t step) {
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t lo = d > nb ? (uint32_t)(d - nb) : 0u;
-    uint32_t hi = d < na ? (uint32_t)d : na;
+    uint32_t lo = max(d > nb ? (uint32_t)(d - nb) : 0u, from);
+    uint32_t hi = min(d < na ? (uint32_t)d : na, to);
     if (step > 0 && hi - lo > 32u * step) {
         const int64_t first = (int64_t)guess - 16 * (int64_t)step;
         const int64_t i = first + (int64_t)(lane + 1) * step;
@@ -178,28 +179,38 @@ __device__ __forceinline__ void merge_tile(const Stage &s, const uint32_t *skb, 
     // left list then always goes first against the right look-ahead element (the
     // merge path put every remaining left element at or below it), and no step
     // can find both ranges exhausted (each step consumes one of the thread's
-    // elements).  The next key of each list is loaded before the comparison, so
-    // the loads are off the step-to-step dependency chain.
+    // elements).  The walk only notes which steps went left and which matched; a lane
+    // has few matches, but at nearly every step some lane of the warp has one, so the
+    // products follow in a loop over the matches (22.6 M entries, synchronous call:
+    // 97.3 us with the products inside the walk, 93.3 so).
     constexpr uint32_t NOKEY = 0xffffffffu;
     uint32_t i = lo, j = d - lo;
     const uint32_t steps = min((uint32_t)CMP_IPT, n - d);
     uint32_t x = i < s.na ? ka[i] : NOKEY, y = j < s.nbx ? kb[j] : NOKEY;
-    for (uint32_t it = 0; it < steps; it++) {
-        const uint32_t xn = i + 1 < s.na ? ka[i + 1] : NOKEY;
-        const uint32_t yn = j + 1 < s.nbx ? kb[j + 1] : NOKEY;
-        if (x == y && x != NOKEY) {
-            float p, e;
-            two_prod(va[i], vb[j], p, e);
-            ff_add(acc, p);
-            acc.lo = __fadd_rn(acc.lo, e);
+    uint32_t left = 0, hit = 0;  // bit t: step t
+#pragma unroll
+    for (uint32_t t = 0; t < (uint32_t)CMP_IPT; t++) {
+        if (t < steps) {
+            const uint32_t xn = i + 1 < s.na ? ka[i + 1] : NOKEY;
+            const uint32_t yn = j + 1 < s.nbx ? kb[j + 1] : NOKEY;
+            if (x == y && x != NOKEY) hit |= 1u << t;
+            if (x <= y) {  // ties go to the left list
+                left |= 1u << t;
+                i++;
+                x = xn;
+            } else {
+                j++;
+                y = yn;
+            }
         }
-        if (x <= y) {  // ties go to the left list
-            i++;
-            x = xn;
-        } else {
-            j++;
-            y = yn;
-        }
+    }
+    while (hit) {
+        const uint32_t t = __ffs(hit) - 1, l = __popc(left & ((1u << t) - 1u));
+        hit &= hit - 1u;
+        float p, e;
+        two_prod(va[lo + l], vb[d - lo + t - l], p, e);
+        ff_add(acc, p);
+        acc.lo = __fadd_rn(acc.lo, e);
     }
 }
 
@@ -277,11 +288,15 @@ __device__ __forceinline__ void producer_drain(Pipe &pp, uint64_t issued, uint32
                                 CMP_DRAIN);
 }
 
-// Producer of one pair: the run's splits are in shared memory (split[r] = left
-// split of tile t_begin + r).
+// Producer of one pair: i0, i1 are the left splits at the start and the end of the run's
+// first tile.  The end of each later tile is searched for from its start, with the last
+// tile's share of left elements as the guess: two rounds of probes near what the copies
+// read anyway, while the copies before it are in flight.  (With all of a CTA's boundaries
+// searched before its first copy, each over the whole lists, the synchronous call on
+// 22.6 M entries took 117.6 us; so, 97.3.)
 __device__ __forceinline__ void produce_one(const uint32_t *Ak, const float *Av, uint32_t na,
                                             const uint32_t *Bk, const float *Bv, uint32_t nb,
-                                            const uint32_t *split, uint64_t t_begin,
+                                            uint32_t i0, uint32_t i1, uint64_t t_begin,
                                             uint64_t t_end, Pipe &pp, uint8_t *raw,
                                             uint32_t *status) {
     const uint32_t lane = threadIdx.x & 31;
@@ -296,16 +311,23 @@ __device__ __forceinline__ void produce_one(const uint32_t *Ak, const float *Av,
             failed = true;
             break;
         }
+        const uint64_t d1 = min((t + 1) * (uint64_t)CMP_TILE, total);
         if (lane == 0) {
-            const uint64_t d0 = t * (uint64_t)CMP_TILE, d1 = min(d0 + CMP_TILE, total);
-            const uint32_t i0 = split[rel], i1 = split[rel + 1];
             issue_stage(pp, s, t, [&](bool issue) {
-                return tile_ranges(Ak, Av, na, Bk, Bv, nb, d0, i0, d1, i1, stage_keys(raw, s),
-                                   stage_vals(raw, s), &pp.full[s], issue);
+                return tile_ranges(Ak, Av, na, Bk, Bv, nb, t * (uint64_t)CMP_TILE, i0, d1, i1,
+                                   stage_keys(raw, s), stage_vals(raw, s), &pp.full[s], issue);
             });
         }
         __syncwarp();
         issued = rel + 1;
+        if (t + 1 < t_end) {
+            const uint64_t d2 = min(d1 + CMP_TILE, total);
+            const uint32_t to = (uint32_t)min((uint64_t)i1 + (d2 - d1), (uint64_t)na);
+            const uint32_t i2 = warp_merge_path(d2, Ak, na, Bk, nb, i1, to,
+                                                (uint64_t)i1 + (i1 - i0), 16);
+            i0 = i1;
+            i1 = i2;
+        }
     }
     if (failed || pp.fail) producer_drain(pp, issued, status);
 }
@@ -387,23 +409,24 @@ __global__ void __launch_bounds__(CMP_THREADS) k_compare(
     uint32_t per, uint32_t first_wait_limit, FF *partial) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ Pipe pp;
-    __shared__ uint32_t s_split[CMP_MAX_RUN + 1], s_status;
+    __shared__ uint32_t s_split[2], s_status;
     __shared__ FF s_final[CMP_CONSUMERS];
     if (threadIdx.x == 0) s_status = DEV_OK;
     const uint64_t total = (uint64_t)na + nb;
     const uint64_t t_begin = (uint64_t)blockIdx.x * per;
     const uint64_t t_end = min((uint64_t)ntiles, t_begin + per);
-    // the splits of this run's boundaries t_begin .. t_end, all warps at once
+    // the splits at both ends of the run's first tile, a warp each
     const uint32_t warp = threadIdx.x >> 5;
-    for (uint64_t b = warp; t_begin < t_end && b <= t_end - t_begin; b += CMP_THREADS / 32) {
-        const uint64_t d = min((t_begin + b) * (uint64_t)CMP_TILE, total);
-        const uint32_t i = warp_merge_path(d, Ak, na, Bk, nb, split_guess(d, na, nb), 64);
-        if ((threadIdx.x & 31) == 0) s_split[b] = i;
+    if (t_begin < t_end && (warp == 0 || warp == CMP_CONSUMERS)) {
+        const uint64_t d = min((t_begin + (warp == 0)) * (uint64_t)CMP_TILE, total);
+        const uint32_t i = warp_merge_path(d, Ak, na, Bk, nb, 0u, na, split_guess(d, na, nb), 64);
+        if ((threadIdx.x & 31) == 0) s_split[warp == 0] = i;
     }
     pipe_init(pp);  // (its barrier also publishes the splits)
     if (threadIdx.x >= CMP_CONSUMER_THREADS) {
         if (t_begin < t_end)
-            produce_one(Ak, Av, na, Bk, Bv, nb, s_split, t_begin, t_end, pp, smem_raw, &s_status);
+            produce_one(Ak, Av, na, Bk, Bv, nb, s_split[0], s_split[1], t_begin, t_end, pp,
+                        smem_raw, &s_status);
         return;
     }
     FF acc = {0.0f, 0.0f};
@@ -491,11 +514,10 @@ cudaError_t compare_launch(cudaStream_t stream, void *scratch, size_t scratch_si
         return launch_next(k_compare_sum, 1, 32, stream, 0u, st, d_out, host_status);
     }
     PHYLO_CHECK(compare_attributes());
-    // two CTAs per SM (three fit): one pair's split searches and the last CTA's
-    // combine cost less over fewer, longer runs (synchronous call on 6.6 M entries:
-    // 0.045 ms against 0.053 with three); at most CMP_MAX_RUN tiles each
+    // three CTAs per SM, as many as fit: synchronous calls on 6.8 M / 22.6 M entries took
+    // 53.6 / 90.0 us, with two 52.5 / 93.3; at most CMP_MAX_RUN tiles each
     const uint32_t sms = (uint32_t)device_sm_count();
-    uint32_t grid = min(ntiles, min(2u * sms, CMP_MIN_CAP));
+    uint32_t grid = min(ntiles, min(3u * sms, CMP_MIN_CAP));
     uint32_t per = (uint32_t)div_up(ntiles, grid);
     if (per > CMP_MAX_RUN) per = CMP_MAX_RUN;
     grid = (uint32_t)div_up(ntiles, per);
