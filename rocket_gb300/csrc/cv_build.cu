@@ -434,7 +434,7 @@ __device__ __forceinline__ uint32_t word_candidates(const BuildArgs &a, int p, u
 
 // Candidates and seen (K-1)-mers per chunk of bitmap words: each of the CTA's warps has
 // warp_words(a) consecutive ones, wpt per lane (8 for the sparse bitmaps of protein K =
-// 7), or 32, 8 or 2 of them with 1, 4 or 16 lanes to a word (see chunk_words).
+// 7), or 32, 8 or 2 of them with 1, 4 or 16 lanes to a word (see chunk_lanes).
 // grid = (NCH + table blocks, B).  With compact (K-2)-mer tables also zeroes the entries
 // in use, which k_c0_scatter counts in.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
