@@ -194,7 +194,10 @@ static int compare_and_wait(cudaStream_t st, Launch launch) {
     uint32_t status = DEV_WAIT_TIMEOUT;
     const bool direct = device_uses_host_memory();
     const cudaError_t e = launch(&d_status, direct ? &status : nullptr);
-    if (e != cudaSuccess) return (int)e;
+    if (e != cudaSuccess) {
+        if (direct) cudaStreamSynchronize(st);  // what was queued may still write to status
+        return (int)e;
+    }
     if (direct) PHYLO_CHECK(cudaStreamSynchronize(st));
     else PHYLO_CHECK(last_status(d_status, st, &status));
     if (status) {

@@ -256,6 +256,8 @@ class BatchBuilder:
             start.record(stream)
             self._side.wait_event(start)
             streams.append(self._side)
+            # freed (also by an exception) only behind the side stream's work
+            d_rel.record_stream(self._side)
         per = np.minimum(8 * lens + 65536, key_limit(self.alphabet, self.k))
         cands = [int(per[f:f + b].sum()) for f, b in batches]
         for slot, st in enumerate(streams):  # scratch for the largest batch of each stream
@@ -364,8 +366,6 @@ class BatchBuilder:
             done = torch.cuda.Event()
             done.record(self._side)
             stream.wait_event(done)
-            # the offsets stay alive until the side stream has finished with them
-            d_rel.record_stream(self._side)
 
 
 def upload_proteomes(data: np.ndarray, device=None, pinned: Optional[torch.Tensor] = None,

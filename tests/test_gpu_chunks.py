@@ -7,6 +7,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 from oracle import oracle as O
+from rocket_gb300 import _native
 from rocket_gb300.engine import BatchBuilder
 
 from gpu_helpers import build_gpu, ulp_diff
@@ -110,3 +111,39 @@ def test_runs_of_tiles(kind, n):
     exact = O.compare_fp64(lk.view(np.uint32), lv, rk.view(np.uint32), rv)
     got = compare_gpu(lk, lv, rk, rv, slot_layout=True)
     assert abs(got - exact) <= 5e-13 * abs(exact)
+
+
+# The chained launches in a graph: replays give the call's bits, also after the inputs
+# have changed in place.
+@pytest.mark.parametrize("n", [0, 40, 300000])
+def test_compare_in_a_graph(n):
+    L = _native.load()
+    rng = np.random.default_rng(n)
+    dev = {}
+    for side in "ab":
+        keys = np.sort(rng.choice(3 * n + 1, n, replace=False)).astype(np.int32)
+        dev[side] = [torch.from_numpy(keys).cuda(),
+                     torch.from_numpy(rng.random(n, dtype=np.float32)).cuda()]
+    scratch = torch.empty(1 << 20, dtype=torch.uint8, device="cuda")
+    out = torch.full((1,), -1.0, dtype=torch.float64, device="cuda")
+
+    def call():
+        (ka, va), (kb, vb) = dev["a"], dev["b"]
+        _native.check(L.phyloComparePairAsync(
+            torch.cuda.current_stream().cuda_stream, scratch.data_ptr(), scratch.numel(),
+            ka.data_ptr(), va.data_ptr(), n, kb.data_ptr(), vb.data_ptr(), n, out.data_ptr()))
+
+    call()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call()
+    for _ in range(3):
+        if n:
+            dev["a"][1].mul_(0.5)
+        call()
+        want = out.item()
+        out.fill_(-1.0)
+        g.replay()
+        torch.cuda.synchronize()
+        assert out.item() == want
