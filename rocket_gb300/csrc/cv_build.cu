@@ -416,6 +416,8 @@ __global__ void __launch_bounds__(COUNT_THREADS) k_count(BuildArgs a) {
     }
 }
 
+constexpr int MAX_WPT = 8;  // bitmap words per thread of the candidate passes, or one
+
 // Consecutive bitmap words of a warp of the candidate passes.
 __device__ __forceinline__ uint32_t warp_words(const BuildArgs &a) { return a.wlanes * a.wpt; }
 
@@ -433,10 +435,13 @@ __device__ __forceinline__ uint32_t word_candidates(const BuildArgs &a, int p, u
 }
 
 // Candidates and seen (K-1)-mers per chunk of bitmap words: each of the CTA's warps has
-// warp_words(a) consecutive ones, wpt per lane (8 for the sparse bitmaps of protein K =
-// 7), or 32, 8 or 2 of them with 1, 4 or 16 lanes to a word (see chunk_lanes).
-// grid = (NCH + table blocks, B).  With compact (K-2)-mer tables also zeroes the entries
+// warp_words(a) consecutive ones, 32, 8 or 2 of them with 1, 4 or 16 lanes to a word (see
+// chunk_lanes); or, WIDE, for the sparse bitmaps of protein K = 7, MAX_WPT times 32, a lane
+// taking every 32nd, and only the warps' totals are kept (12 uneven proteomes: 195 -> 148
+// us against MAX_WPT neighbouring words per lane and a count per word; k_cand_offsets, which
+// then reads coalesced too, 400 -> 365).  grid = (NCH + table blocks, B).  With compact (K-2)-mer tables also zeroes the entries
 // in use, which k_c0_scatter counts in.
+template <bool WIDE>
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
     previous_kernel_done();
     const int p = blockIdx.y, c = blockIdx.x;
@@ -446,11 +451,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
     }
     const uint64_t nw = a.T1s / 32;
     const uint32_t lane = threadIdx.x & 31u, shared = 32u / a.wlanes;  // lanes to a word
-    const uint64_t wd0 = ((uint64_t)c * (CHUNK_THREADS / 32) + threadIdx.x / 32) * warp_words(a) +
-                         lane / shared * a.wpt;
+    const uint64_t wd0 =
+        ((uint64_t)c * (CHUNK_THREADS / 32) + threadIdx.x / 32) * warp_words(a) + lane / shared;
     uint32_t s = 0, n = 0;
-    for (uint32_t i = 0; i < a.wpt; i++) {
-        const uint64_t wd = wd0 + i;
+    for (uint32_t i = 0; i < (WIDE ? MAX_WPT : 1); i++) {
+        const uint64_t wd = wd0 + 32 * i;
         uint32_t bits = 0, sw = 0;
         if (wd < nw) {
             bits = a.seen1[(uint64_t)p * nw + wd];
@@ -459,6 +464,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
         }
         s += sw;
         n += __popc(bits);
+        if (WIDE) continue;
         for (uint32_t d = 1; d < shared; d <<= 1) sw += __shfl_xor_sync(0xffffffffu, sw, d);
         if (wd < nw && lane % shared == 0) a.word_cand[(uint64_t)p * nw + wd] = sw;
     }
@@ -468,6 +474,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_count(BuildArgs a) {
     if ((threadIdx.x & 31) == 0) {
         ws[threadIdx.x >> 5] = s;
         wn[threadIdx.x >> 5] = n;
+        if (WIDE)
+            a.warp_cs[((uint64_t)p * a.NCH + c) * (CHUNK_THREADS / 32) + (threadIdx.x >> 5)] =
+                make_uint2(s, n);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -548,8 +557,6 @@ __global__ void __launch_bounds__(CSCAN_THREADS) k_cand_scan(BuildArgs a) {
     }
 }
 
-constexpr int MAX_WPT = 8;  // bitmap words per thread of the chunk kernels, at most
-
 __device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v) {
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
@@ -575,10 +582,11 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t i) {
 // coff[p][q] = candidate offset of seen (K-1)-mer q within proteome p (entries
 // of unseen q are not written); cq = the key q * A + b of every candidate (b over
 // the right-extension mask of q's suffix, ascending), c0a zeroed.  A warp owns a
-// contiguous run of bitmap words, wpt per lane of its first wlanes, and their candidates;
-// these and the seen (K-1)-mers start at the exclusive scans of the word_cand sums and
-// the words' populations (one scan of packed pairs; with compact tables pw1 gets the
-// ranks of the words that hold any).  The warp
+// contiguous run of bitmap words, one per lane of its first wlanes (WIDE: MAX_WPT times
+// 32), and their candidates; these and the seen (K-1)-mers start at the exclusive scans of
+// the word_cand sums and the words' populations (one scan of packed pairs; WIDE: at the
+// totals of the warps before).  With compact tables pw1 gets the ranks of the words that
+// hold any.  The warp
 // processes its run together: its seen (K-1)-mers, 32 at a time in order (each lane
 // finds its own by a search over the scan of the words' populations), load
 // their masks together; a warp scan of the mask populations places their
@@ -589,9 +597,9 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t i) {
 // the sparse words of K = 7; finding each key's (K-1)-mer by a search over the
 // scan cost about three times the instructions of the stage.)
 // grid = (NCH, B)
+template <bool WIDE>
 __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
     previous_kernel_done();
-    __shared__ uint64_t sw[CHUNK_THREADS / 32 + 1];
     __shared__ uint32_t s_stage[CHUNK_THREADS / 32][32 * 21];  // keys of 32 seen (K-1)-mers (A <= 21)
     uint32_t *stage = s_stage[threadIdx.x >> 5];
     const int p = blockIdx.y, c = blockIdx.x;
@@ -601,36 +609,48 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_cand_offsets(BuildArgs a) {
     const uint32_t *seen = a.seen1 + (uint64_t)p * nw;
     const uint64_t wbeg =
         ((uint64_t)c * (CHUNK_THREADS / 32) + threadIdx.x / 32) * warp_words(a);
-    const uint64_t wd0 = wbeg + lane * a.wpt;
-    uint32_t s = 0, npop = 0;
-    for (uint32_t i = 0; i < a.wpt && lane < a.wlanes && wd0 + i < nw; i++) {
-        s += a.word_cand[(uint64_t)p * nw + wd0 + i];
-        npop += __popc(seen[wd0 + i]);
+    // the warp's candidates [run, r1) of the proteome, and the rank P of its first seen
+    // (K-1)-mer among the batch's
+    uint32_t run =
+        (uint32_t)(a.chunk_cand_off[pc] - a.chunk_cand_off[(uint64_t)p * a.NCH]);
+    uint32_t P = a.chunk_seen_off[pc], r1;
+    if constexpr (WIDE) {
+        const uint32_t warp = threadIdx.x >> 5;
+        const uint2 t =
+            lane <= warp ? a.warp_cs[pc * (CHUNK_THREADS / 32) + lane] : make_uint2(0u, 0u);
+        run += __reduce_add_sync(0xffffffffu, lane < warp ? t.x : 0u);
+        P += __reduce_add_sync(0xffffffffu, lane < warp ? t.y : 0u);
+        r1 = run + __shfl_sync(0xffffffffu, t.x, (int)warp);
+    } else {
+        __shared__ uint64_t sw[CHUNK_THREADS / 32 + 1];
+        uint32_t s = 0, npop = 0;
+        if (lane < a.wlanes && wbeg + lane < nw) {
+            s = a.word_cand[(uint64_t)p * nw + wbeg + lane];
+            npop = __popc(seen[wbeg + lane]);
+        }
+        uint64_t tot;
+        const uint64_t ex =
+            block_excl_scan_u64<CHUNK_THREADS>((uint64_t)npop << 32 | s, sw, &tot);
+        r1 = run + __shfl_sync(0xffffffffu, (uint32_t)ex + s, 31);
+        run += __shfl_sync(0xffffffffu, (uint32_t)ex, 0);
+        P += __shfl_sync(0xffffffffu, (uint32_t)(ex >> 32), 0);
     }
-    uint64_t tot;
-    const uint64_t ex = block_excl_scan_u64<CHUNK_THREADS>((uint64_t)npop << 32 | s, sw, &tot);
-    const uint32_t run0 =
-        (uint32_t)(a.chunk_cand_off[pc] - a.chunk_cand_off[(uint64_t)p * a.NCH]) + (uint32_t)ex;
-    // rank of the warp's first seen (K-1)-mer among the batch's
-    uint32_t P = a.chunk_seen_off[pc] + __shfl_sync(0xffffffffu, (uint32_t)(ex >> 32), 0);
     const uint64_t gb = a.cbase[p];
-    uint32_t run = __shfl_sync(0xffffffffu, run0, 0);
-    const uint32_t r1 = __shfl_sync(0xffffffffu, run0 + s, 31);
     // zero this warp's K-mer count slots (coalesced)
     for (uint64_t i = gb + run + lane; i < gb + r1 && i < a.cand_cap; i += 32) a.c0a[i] = 0u;
     // the warp's words [wbeg, wend), loaded up front (coalesced), lane l holding word
     // wbeg + 32 t + l of group t; the seen (K-1)-mers of a group are taken 32 at a time
     const uint64_t wend = min(wbeg + warp_words(a), nw);
     const uint32_t A = a.A;
-    uint32_t wreg[MAX_WPT];
+    constexpr int WPT = WIDE ? MAX_WPT : 1;
+    uint32_t wreg[WPT];
 #pragma unroll
-    for (int t = 0; t < MAX_WPT; t++) {
+    for (int t = 0; t < WPT; t++) {
         const uint64_t w = wbeg + 32 * t + lane;
-        wreg[t] = ((uint32_t)t < a.wpt && w < wend) ? seen[w] : 0u;
+        wreg[t] = w < wend ? seen[w] : 0u;
     }
 #pragma unroll
-    for (int t = 0; t < MAX_WPT; t++) {
-        if ((uint32_t)t >= a.wpt) break;
+    for (int t = 0; t < WPT; t++) {
         const uint32_t wbits = wreg[t];
         const uint32_t wincl = warp_incl_scan_u32(__popc(wbits));
         const uint32_t nseen = __shfl_sync(0xffffffffu, wincl, 31);
@@ -1008,9 +1028,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
     previous_kernel_done();
     const int p = blockIdx.y;
     const uint64_t nw = a.T1s / 32;
-    const uint64_t wd0 = ((uint64_t)blockIdx.x * CHUNK_THREADS + threadIdx.x) * a.wpt;
+    const uint64_t wd0 = (uint64_t)blockIdx.x * CHUNK_THREADS * a.wpt + threadIdx.x;
     for (uint32_t i = 0; i < a.wpt; i++) {
-        const uint64_t wd = wd0 + i;
+        const uint64_t wd = wd0 + i * CHUNK_THREADS;
         if (wd >= nw) break;
         uint32_t bits = a.seen1[(uint64_t)p * nw + wd];
         while (bits) {
@@ -1210,7 +1230,8 @@ static void build_layout(const BuildGeometry &g, int B, uint64_t cand_cap, Build
     if (compact2) take(r.c2, r.cap2);
     take(r.pw1, compact ? nw1 : 0);
     take(r.p1_total, 1);
-    take(r.word_cand, nw1);
+    take(r.word_cand, g.wpt > 1 ? 0 : nw1);
+    take(r.warp_cs, g.wpt > 1 ? nc * (CHUNK_THREADS / 32) : 0);
     take(r.pw2, compact2 ? nw2 : 0);
     take(r.p2_partials, compact2 ? bitmap_prefix_partials(nw2) : 0);
     take(r.p2_total, 1);
@@ -1283,10 +1304,11 @@ cudaError_t build_plan(BuildArgs &a, cudaStream_t st) {
     if (a.compact2)  // ranks of the seen (K-2)-mers
         PHYLO_CHECK(bitmap_prefix_pairs(a.seen2, a.T2s / 32 * a.B, a.p2_partials, a.pw2,
                                         a.p2_total, st));
-    PHYLO_CHECK(launch_next(k_cand_count, dim3(nch + PROB_BLOCKS + TUPLE_BLOCKS, B), CHUNK_THREADS,
-                            st, a));
+    PHYLO_CHECK(launch_next(a.wpt > 1 ? k_cand_count<true> : k_cand_count<false>,
+                            dim3(nch + PROB_BLOCKS + TUPLE_BLOCKS, B), CHUNK_THREADS, st, a));
     PHYLO_CHECK(launch_next(k_cand_scan, 1, CSCAN_THREADS, st, a));
-    PHYLO_CHECK(launch_next(k_cand_offsets, dim3(nch, B), CHUNK_THREADS, st, a));
+    PHYLO_CHECK(launch_next(a.wpt > 1 ? k_cand_offsets<true> : k_cand_offsets<false>, dim3(nch, B),
+                            CHUNK_THREADS, st, a));
     PHYLO_CHECK(launch_next(k_c0_scatter, grid_seq, COUNT_THREADS, st, a));
     PHYLO_CHECK(launch_next(k_alpha, (unsigned)(a.cand_cap / ALPHA_TILE), CHUNK_THREADS, st, a));
     PHYLO_CHECK(launch_next(k_norm, B, NORM_THREADS, st, a));

@@ -79,7 +79,8 @@ struct BuildArgs {
     uint2 *pw1;               // [B * T1s / 32]: {set bits of seen1 before the word, the word}
     uint64_t *p1_total;
     uint32_t *seen1;          // [B][T1s / 32]: bitmap of the seen (K-1)-mers
-    uint32_t *word_cand;      // [B][T1s / 32]: candidates of each bitmap word
+    uint32_t *word_cand;      // [B][T1s / 32]: candidates of each bitmap word (wpt = 1), or
+    uint2 *warp_cs;           // [B * NCH][warps]: candidates, seen (K-1)-mers of each warp
     // (K-2)-mer counts: dense [B][T2], or, when `compact2` (beyond 2^20 entries),
     // one entry per seen (K-2)-mer of the batch, at its rank in seen2 (via pw2)
     uint32_t *c2;

@@ -49,11 +49,11 @@ def test_short_and_long_single_proteomes(n):
 # Batches on both sides of the lines between 2, 8 and 32 lanes with words: 32 lanes from
 # 1,500 chunks on, which at K = 6 (499 each) takes 4 proteomes and 8 lanes below; at K = 5
 # 8 lanes from 16 proteomes (95 chunks each), over DNA at K = 10 from 12 (128 each), and 2
-# lanes below; at K = 3 and 4 a few chunks in all.
+# lanes below; at K = 3 and 4 a few chunks in all.  K = 7: eight words per lane.
 @pytest.mark.parametrize("alphabet,k,batch", [
     ("protein", 3, 1), ("protein", 4, 5), ("protein", 5, 1), ("protein", 5, 4),
     ("protein", 5, 15), ("protein", 5, 16), ("protein", 6, 1), ("protein", 6, 3),
-    ("protein", 6, 4), ("DNA", 3, 2), ("DNA", 8, 3), ("DNA", 10, 2), ("DNA", 10, 3),
+    ("protein", 6, 4), ("protein", 7, 1), ("protein", 7, 3), ("DNA", 3, 2), ("DNA", 8, 3), ("DNA", 10, 2), ("DNA", 10, 3),
     ("DNA", 10, 12)])
 def test_batches_over_every_chunk_size(alphabet, k, batch):
     letters = AMINO if alphabet == "protein" else BASES
