@@ -1023,12 +1023,16 @@ __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
 // one or two atomics per seen (K-1)-mer instead of one per written key.  The
 // marked set is a superset of the written keys (a candidate whose alpha is 0 is
 // marked but not written), which is all a key-rank bitmap needs: ranks stay
-// strictly increasing over the written keys.  grid = (words / (CHUNK_THREADS * wpt), B)
+// strictly increasing over the written keys.  grid = (words / (CHUNK_THREADS * wpt), B), or
+// WIDE (K = 7) its transpose: the bitmap (225 MB) is larger than L2 there, and the batch's
+// proteomes mark the same stretch of it at a time (12 uneven proteomes: 203 -> 162 us; at K =
+// 6, where it stays in L2, they would only meet in its words: 111 -> 120).
+template <bool WIDE>
 __global__ void __launch_bounds__(CHUNK_THREADS) k_union_mark(BuildArgs a) {
     previous_kernel_done();
-    const int p = blockIdx.y;
+    const int p = WIDE ? blockIdx.x : blockIdx.y;
     const uint64_t nw = a.T1s / 32;
-    const uint64_t wd0 = (uint64_t)blockIdx.x * CHUNK_THREADS * a.wpt + threadIdx.x;
+    const uint64_t wd0 = (uint64_t)(WIDE ? blockIdx.y : blockIdx.x) * CHUNK_THREADS * a.wpt + threadIdx.x;
     for (uint32_t i = 0; i < a.wpt; i++) {
         const uint64_t wd = wd0 + i * CHUNK_THREADS;
         if (wd >= nw) break;
@@ -1323,11 +1327,13 @@ cudaError_t build_emit(BuildArgs &a, cudaStream_t st) {
         a.pad_blocks = (unsigned)min(div_up(a.single_cap ? a.single_cap : 1, 8 * CHUNK_THREADS),
                                      (uint64_t)device_sm_count() * 8);
     PHYLO_CHECK(launch_next(k_compact, (unsigned)(ncta + a.pad_blocks), CHUNK_THREADS, st, a));
-    if (a.union_bits)
-        PHYLO_CHECK(launch_next(k_union_mark,
-                                dim3((unsigned)div_up(a.T1s / 32, (uint64_t)CHUNK_THREADS * a.wpt),
-                                     (unsigned)a.B),
-                                CHUNK_THREADS, st, a));
+    if (a.union_bits) {
+        const unsigned words = (unsigned)div_up(a.T1s / 32, (uint64_t)CHUNK_THREADS * a.wpt);
+        PHYLO_CHECK(a.wpt > 1 ? launch_next(k_union_mark<true>, dim3((unsigned)a.B, words),
+                                            CHUNK_THREADS, st, a)
+                              : launch_next(k_union_mark<false>, dim3(words, (unsigned)a.B),
+                                            CHUNK_THREADS, st, a));
+    }
     return cudaGetLastError();
 }
 
