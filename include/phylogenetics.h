@@ -222,7 +222,8 @@ int phyloPairsLaunch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_val
  * part, tile, s0, s1 and two unused: windows [w0, w1), w0 < w1, of the segment [s0, s1),
  * the parts of a segment covering it in order.  Each part takes the FP32 accumulator
  * runs (of `fold` slots per lane) that begin in its windows, so the sums are those of
- * the unsplit segment. */
+ * the unsplit segment.  tile_rows 16, or 8 or 4 where no part has more rows than that (the
+ * partial blocks stay 16 x tile_cols). */
 int phyloPairsLaunchParts(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_values,
                           uintptr_t d_row_vec_off, uintptr_t d_row_roff, uintptr_t d_col_keys,
                           uintptr_t d_col_values, uintptr_t d_col_vec_off, uintptr_t d_col_roff,

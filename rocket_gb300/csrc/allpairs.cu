@@ -37,7 +37,8 @@ namespace phylo {
 // spread random keys over all eight bank groups and conflicted more: all pairs of 64
 // uniform proteomes of 1,500 proteins took 500 M load wavefronts, 282 M of them conflicts,
 // against 381 M and 163 M, and 2.55 ms against 2.10 with the packed FP32 FMAs and the
-// row scatter below.)  One extra record (index W) stays zero for masked lanes.
+// row scatter below.)  One extra record (index W) stays zero for masked lanes.  Parts of
+// few rows have records of 32 or 16 bytes (ap_parts_kernel).
 constexpr uint32_t D_REC = 64;  // bytes per key record
 
 // acc (two FP32 sums) += record values * b, each as __fmaf_rn
@@ -50,23 +51,26 @@ __device__ __forceinline__ uint64_t pack2(float x, float y) {
     return r;
 }
 
-// Adds record * b to the lane's sums.  at: offset in the table of the record's chunk
-// lane & 3 (records start at multiples of 64); chunk t ^ (lane & 3) goes to sums
-// 4 t .. 4 t + 3.
+// Adds record * b to the lane's sums.  A record of ROWS row values is ROWS / 4 chunks of
+// 16 bytes; at: offset in the table of the record's chunk lane % (ROWS / 4) (records start
+// at multiples of their size); chunk t ^ (lane % (ROWS / 4)) goes to sums 4 t .. 4 t + 3.
+template <int ROWS>
 __device__ __forceinline__ void fma_record(const unsigned char *table, uint32_t at, float b,
-                                           uint64_t (&acc)[8]) {
+                                           uint64_t (&acc)[ROWS / 2]) {
     const uint64_t bb = pack2(b, b);
 #pragma unroll
-    for (uint32_t t = 0; t < 4; t++) {
+    for (uint32_t t = 0; t < ROWS / 4; t++) {
         const float4 v = *reinterpret_cast<const float4 *>(table + (at ^ (16u * t)));
         fma2(acc[2 * t], pack2(v.x, v.y), bb);
         fma2(acc[2 * t + 1], pack2(v.z, v.w), bb);
     }
 }
 
-__device__ __forceinline__ void fold_pairs(uint64_t (&acc)[8], float (&hi)[16], float (&lo)[16]) {
+template <int ROWS>
+__device__ __forceinline__ void fold_pairs(uint64_t (&acc)[ROWS / 2], float (&hi)[ROWS],
+                                           float (&lo)[ROWS]) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < ROWS / 2; i++) {
         float x[2];
         asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(acc[i]));
         acc[i] = 0ull;
@@ -82,11 +86,12 @@ __device__ __forceinline__ void fold_pairs(uint64_t (&acc)[8], float (&hi)[16], 
 
 // The lane's sums of rows 8 half .. 8 half + 7 (see fma_record) to stage[row of the
 // half * stride + lane].
-__device__ __forceinline__ void stage_sums(const float (&hi)[16], const float (&lo)[16], FF *stage,
-                                           uint32_t stride, uint32_t half) {
+template <int ROWS>
+__device__ __forceinline__ void stage_sums(const float (&hi)[ROWS], const float (&lo)[ROWS],
+                                           FF *stage, uint32_t stride, uint32_t half) {
 #pragma unroll
-    for (uint32_t t = 0; t < 4; t++) {
-        const uint32_t ch = t ^ (threadIdx.x & 3u);  // rows 4 ch .. 4 ch + 3
+    for (uint32_t t = 0; t < ROWS / 4; t++) {
+        const uint32_t ch = t ^ (threadIdx.x & (ROWS / 4 - 1u));  // rows 4 ch .. 4 ch + 3
         if (ch >> 1 == half) {
 #pragma unroll
             for (uint32_t c = 0; c < 4; c++)
@@ -149,18 +154,18 @@ __device__ __forceinline__ void assign_lanes(const ApItem &item, uint32_t *s_lan
 // Sums of the lanes of each column, in lane order, into the item's partial block
 // (rows x tj float pairs).  The sums pass through `stage` (8 rows x THREADS float
 // pairs: the idle cp.async ring), eight rows at a time.
-template <int THREADS>
-__device__ __forceinline__ void combine_lanes(const float (&hi)[16], const float (&lo)[16],
+template <int THREADS, int ROWS>
+__device__ __forceinline__ void combine_lanes(const float (&hi)[ROWS], const float (&lo)[ROWS],
                                               FF *stage, FF *dst, uint32_t tj, bool has_col,
                                               uint32_t jcol, uint32_t l0, uint32_t q,
                                               uint32_t lpc) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < (ROWS + 7) / 8; h++) {
         __syncthreads();
-        stage_sums(hi, lo, stage, THREADS, h);
+        stage_sums<ROWS>(hi, lo, stage, THREADS, h);
         __syncthreads();
         if (has_col) {
-            for (uint32_t i = q; i < 8; i += lpc) {
+            for (uint32_t i = q; i < (ROWS < 8 ? ROWS : 8); i += lpc) {
                 FF v = stage[i * THREADS + l0];
                 for (uint32_t m = 1; m < lpc; m++) v = ff_merge(v, stage[i * THREADS + l0 + m]);
                 dst[(8 * h + i) * tj + jcol] = v;
@@ -230,17 +235,18 @@ __device__ __forceinline__ uint32_t visits_before(const uint32_t *__restrict__ c
 // instead of read from the zero record (7.37), a deeper column ring (6.95), 512- or
 // 1,024-key tables scattered by producer warps while the others gather (9.0, 7.9: every
 // end of a narrower window makes each lane look at a partly used group once more).
-template <int THREADS, int MINB, int LPC, bool PARTS>
+template <int THREADS, int MINB, int LPC, bool PARTS, int ROWS>
 __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
     constexpr int TJ = THREADS / LPC;            // column vectors per item
-    constexpr uint32_t SL = THREADS / AP_TI;     // threads per row
-    constexpr uint32_t RPG = AP_TI / (THREADS / 128);  // rows per warp group
+    constexpr uint32_t SL = THREADS / ROWS;     // threads per row
+    constexpr uint32_t RPG = ROWS / (THREADS / 128);  // rows per warp group
     constexpr int RING = ring_depth(THREADS);
+    constexpr uint32_t REC = 4 * ROWS;           // bytes per key record
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t W = 1u << a.wshift, wmask = W - 1u;
     // the table (W + 1 records) and the column ring
     float *D = reinterpret_cast<float *>(smem);
-    uint4 *ring_k = reinterpret_cast<uint4 *>(smem + (size_t)(W + 1) * D_REC);
+    uint4 *ring_k = reinterpret_cast<uint4 *>(smem + (size_t)(W + 1) * REC);
     float4 *ring_v = reinterpret_cast<float4 *>(ring_k + RING * THREADS);
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_lane0[TJ + 1];
@@ -248,10 +254,10 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
     const uint32_t wg = threadIdx.x / 128;
     const uint32_t rr = wg * RPG + threadIdx.x % RPG, sl = threadIdx.x % 128 / RPG;
     const uint32_t Rs = a.R + 1;
-    const uint32_t chunk = 16u * (threadIdx.x & 3u);  // of a record, read first
+    const uint32_t chunk = 16u * (threadIdx.x & (ROWS / 4 - 1u));  // of a record, read first
     float *drow = D + rr;  // this thread's row of the records
 
-    for (uint32_t i = threadIdx.x; i < (W + 1) * (D_REC / 16); i += THREADS)
+    for (uint32_t i = threadIdx.x; i < (W + 1) * (REC / 16); i += THREADS)
         reinterpret_cast<float4 *>(smem)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     for (;;) {
@@ -328,12 +334,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
             }
         };
         prefetch_row(r_lo, r_hi);
-        uint64_t acc[8];
-        float hi[16], lo[16];
+        uint64_t acc[ROWS / 2];
+        float hi[ROWS], lo[ROWS];
 #pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = 0ull;
+        for (int i = 0; i < ROWS / 2; i++) acc[i] = 0ull;
 #pragma unroll
-        for (int i = 0; i < 16; i++) hi[i] = lo[i] = 0.0f;
+        for (int i = 0; i < ROWS; i++) hi[i] = lo[i] = 0.0f;
 
         for (uint32_t r = item.w0; r < s1; r++) {
             // scatter window r of row rr: prefetched groups, the rest loaded.  held: window
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
                     for (uint32_t u = 0; u < 4; u++) {
                         const bool in = e + u >= r_lo && e + u < r_hi;
                         off[u] = in ? ks[u] & wmask : W;
-                        if (in) drow[off[u] * AP_TI] = vs[u];
+                        if (in) drow[off[u] * ROWS] = vs[u];
                     }
                     held[2 * k] = off[0] | off[1] << 16;
                     held[2 * k + 1] = off[2] | off[3] << 16;
@@ -366,7 +372,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
                 const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
 #pragma unroll
                 for (uint32_t u = 0; u < 4; u++)
-                    if (e + u < rest_hi) drow[(ks[u] & wmask) * AP_TI] = vs[u];
+                    if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = vs[u];
             }
             // the next window's row entries
             r_lo = r_hi;
@@ -397,12 +403,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
                     for (int u = 0; u < 4; u++) {
                         const uint32_t e = cur + u;
                         const bool ok = e >= first && e < c_hi;
-                        fma_record(smem, chunk + (ok ? ks[u] & wmask : W) * D_REC,
+                        fma_record<ROWS>(smem, chunk + (ok ? ks[u] & wmask : W) * REC,
                                    ok ? vs[u] : 0.0f, acc);
                     }
                     nacc += 4;
                     if (nacc >= (int32_t)a.fold) {
-                        fold_pairs(acc, hi, lo);
+                        fold_pairs<ROWS>(acc, hi, lo);
                         nacc = 0;
                         if (PARTS && r >= item.w1) {
                             cur = AP_DONE;
@@ -431,22 +437,22 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
             // clear window r of row rr
 #pragma unroll
             for (uint32_t k = 0; k < 2 * AP_STAGE; k++) {
-                if ((held[k] & 0xffffu) != W) drow[(held[k] & 0xffffu) * AP_TI] = 0.0f;
-                if (held[k] >> 16 != W) drow[(held[k] >> 16) * AP_TI] = 0.0f;
+                if ((held[k] & 0xffffu) != W) drow[(held[k] & 0xffffu) * ROWS] = 0.0f;
+                if (held[k] >> 16 != W) drow[(held[k] >> 16) * ROWS] = 0.0f;
             }
             for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
                 const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
                 const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
 #pragma unroll
                 for (uint32_t u = 0; u < 4; u++)
-                    if (e + u < rest_hi) drow[(ks[u] & wmask) * AP_TI] = 0.0f;
+                    if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = 0.0f;
             }
             if (PARTS && !more) break;
             bar_sync(1 + (int)wg, 128);
         }
         cp_async_wait_all();
-        fold_pairs(acc, hi, lo);
-        combine_lanes<THREADS>(hi, lo, reinterpret_cast<FF *>(ring_k),
+        fold_pairs<ROWS>(acc, hi, lo);
+        combine_lanes<THREADS, ROWS>(hi, lo, reinterpret_cast<FF *>(ring_k),
                                a.part + (uint64_t)item.part * (AP_TI * TJ), TJ, has_col, jcol, l0,
                                q, lpc);
         if (a.item_cycles && threadIdx.x == 0) a.item_cycles[it] = clock64() - t_start;
@@ -730,27 +736,45 @@ int ap_threads(uint32_t wshift, int tile_rows, int tile_cols) {
     return tile_cols * ap_lpc(tile_cols);
 }
 
-static const void *ap_kernel(uint32_t wshift, int tile_rows, int tile_cols, bool parts) {
+static const void *ap_kernel(uint32_t wshift, int tile_rows, int tile_cols) {
     if (tile_rows == 32)
         return r32_wide(wshift) ? (const void *)k_allpairs32<512, 1>
                                 : (const void *)k_allpairs32<256, 2>;
+    if (tile_cols == 256) return (const void *)k_allpairs<512, 1, 2, false, 16>;
+    if (tile_cols == 128) return (const void *)k_allpairs<512, 1, 4, false, 16>;
+    return tile_cols == 32 ? (const void *)k_allpairs<128, 4, 4, false, 16>
+                           : (const void *)k_allpairs<256, 2, 4, false, 16>;
+}
+
+// The kernels of parts: 16 x 128 and 16 x 256 tiles, and those whose tiles have at most
+// eight or four rows (records of 32 or 16 bytes, so half or a quarter of the loads and
+// FMAs; the row values of a key are added to their own sums in the same order).  160 uneven
+// vectors against 1..4 rows: 8.0 -> 4.0 ms, against 5..8: 8.1 -> 5.0, against 24 (16 and
+// 8, two launches) 14.5 -> 13.6; twelve rows as
+// eight and four 8.7 (16-row records: 8.5).  Two CTAs per SM, with half the ring: 4.5 / 6.8.
+static const void *ap_parts_kernel(int rows, int tile_cols) {
     if (tile_cols == 256)
-        return parts ? (const void *)k_allpairs<512, 1, 2, true>
-                     : (const void *)k_allpairs<512, 1, 2, false>;
-    if (tile_cols == 128)
-        return parts ? (const void *)k_allpairs<512, 1, 4, true>
-                     : (const void *)k_allpairs<512, 1, 4, false>;
-    return tile_cols == 32 ? (const void *)k_allpairs<128, 4, 4, false>
-                           : (const void *)k_allpairs<256, 2, 4, false>;
+        return rows == 16  ? (const void *)k_allpairs<512, 1, 2, true, 16>
+               : rows == 8 ? (const void *)k_allpairs<512, 1, 2, true, 8>
+                           : (const void *)k_allpairs<512, 1, 2, true, 4>;
+    return rows == 16  ? (const void *)k_allpairs<512, 1, 4, true, 16>
+           : rows == 8 ? (const void *)k_allpairs<512, 1, 4, true, 8>
+                       : (const void *)k_allpairs<512, 1, 4, true, 4>;
+}
+
+static size_t ap_parts_smem(uint32_t wshift, int rows) {
+    return (((size_t)1 << wshift) + 1) * 4 * rows + ap_ring_bytes(512);
 }
 
 cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_per_sm) {
     const size_t smem = ap_smem_bytes(wshift, tile_rows, tile_cols);
-    const void *fn = ap_kernel(wshift, tile_rows, tile_cols, false);
+    const void *fn = ap_kernel(wshift, tile_rows, tile_cols);
     PHYLO_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (tile_rows == AP_TI && tile_cols >= 128)
-        PHYLO_CHECK(cudaFuncSetAttribute(ap_kernel(wshift, tile_rows, tile_cols, true),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        for (int rows = 4; rows <= AP_TI; rows *= 2)
+            PHYLO_CHECK(cudaFuncSetAttribute(ap_parts_kernel(rows, tile_cols),
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)ap_parts_smem(wshift, rows)));
     if (ctas_per_sm) {
         int n = 0;
         PHYLO_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -763,8 +787,11 @@ cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_
 cudaError_t ap_launch(const ApArgs &a, int tile_rows, int tile_cols, int grid, cudaStream_t st) {
     ApArgs arg = a;
     void *argv[] = {&arg};
-    return cudaLaunchKernel(ap_kernel(a.wshift, tile_rows, tile_cols, a.subs != nullptr),
-                            dim3(grid), dim3(ap_threads(a.wshift, tile_rows, tile_cols)), argv,
+    if (a.subs)
+        return cudaLaunchKernel(ap_parts_kernel(tile_rows, tile_cols), dim3(grid), dim3(512), argv,
+                                ap_parts_smem(a.wshift, tile_rows), st);
+    return cudaLaunchKernel(ap_kernel(a.wshift, tile_rows, tile_cols), dim3(grid),
+                            dim3(ap_threads(a.wshift, tile_rows, tile_cols)), argv,
                             ap_smem_bytes(a.wshift, tile_rows, tile_cols), st);
 }
 

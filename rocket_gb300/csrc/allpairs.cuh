@@ -56,6 +56,7 @@ size_t ap_smem_bytes(uint32_t wshift, int tile_rows, int tile_cols);
 int ap_max_wshift(int tile_rows, int tile_cols);
 int ap_threads(uint32_t wshift, int tile_rows, int tile_cols);
 cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_per_sm);
+// (parts: tile_rows 16, or 8 or 4 where no part has more rows)
 cudaError_t ap_launch(const ApArgs &a, int tile_rows, int tile_cols, int grid, cudaStream_t st);
 
 // window index: roff[v][r] = number of entries of vector v with key < r << wshift

@@ -511,9 +511,11 @@ static int pairs_launch(uintptr_t stream, uintptr_t d_row_keys, uintptr_t d_row_
                         uintptr_t d_colids, uintptr_t d_items, int num_items, uintptr_t d_counter,
                         uintptr_t d_part, int fold, uintptr_t d_item_cycles, int tile_rows,
                         int tile_cols, int grid, bool parts) {
-    if (!ap_shape_ok(tile_rows, tile_cols) || window_shift < 4 ||
-        window_shift > ap_max_wshift(tile_rows, tile_cols) || num_items < 0 || grid <= 0 ||
-        (parts && (tile_rows != AP_TI || tile_cols < 128)))
+    // parts of at most eight or four rows are parts of 16-row tiles
+    const int shape = parts && (tile_rows == 8 || tile_rows == 4) ? AP_TI : tile_rows;
+    if (!ap_shape_ok(shape, tile_cols) || window_shift < 4 ||
+        window_shift > ap_max_wshift(shape, tile_cols) || num_items < 0 || grid <= 0 ||
+        (parts && (shape != AP_TI || tile_cols < 128)))
         return (int)cudaErrorInvalidValue;
     ApArgs a;
     a.row.keys = (const uint32_t *)d_row_keys;

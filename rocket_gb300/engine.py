@@ -412,6 +412,7 @@ class PairPlan:
     host_part_tiles: np.ndarray = field(default=None)  # int64 [ntiles, 8] with parts
     parts: torch.Tensor = None       # int32 device copies of both
     part_tiles: torch.Tensor = None
+    part_groups: list = field(default_factory=list)  # launches: (first part, parts, rows)
 
 
 @dataclass
@@ -462,7 +463,7 @@ class PairEngine:
         props = torch.cuda.get_device_properties(self.device)
         self.sms = props.multi_processor_count
         self.grid = self.sms * self.ctas_per_sm
-        self.counter = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self.counter = torch.zeros(3, dtype=torch.int32, device=self.device)  # one per launch
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.part = None
         self.launches = 0
@@ -683,7 +684,7 @@ class PairEngine:
                 self.cfg.tile_cols >= 128:
             cut = self._cut_items(S, cost, host_tiles, col_nnz[colids])
             if cut is not None:
-                parts, part_tiles = cut
+                parts, part_tiles, groups = cut
                 nparts = len(parts)
         # one copy to the device: each array from a 16-byte boundary
         arrays = [rowids, colids, host_tiles, items, parts, part_tiles]
@@ -701,12 +702,13 @@ class PairEngine:
             nparts=nparts, host_rowids=rowids, host_colids=colids, host_tiles=host_tiles,
             item_tile=item_tile, item_share=share)
         if cut is not None:
-            plan.host_parts, plan.host_part_tiles = cut
+            plan.host_parts, plan.host_part_tiles = parts, part_tiles
             plan.parts, plan.part_tiles = views[4], views[5]
+            plan.part_groups = groups
         return plan
 
     def _cut_items(self, S, cost, host_tiles, nnz_of_col):
-        """(parts [n, 12], tiles [ntiles, 8]) of a plan of S segments per tile whose items
+        """(parts [n, 12], tiles [ntiles, 8], launches) of a plan of S segments per tile whose items
         are too few to fill the GPU, longest first, or None where no segment is cut.
         ``cost``: of each tile; ``nnz_of_col``: entries of the plan's columns in their
         order, most first."""
@@ -749,7 +751,17 @@ class PairEngine:
         tiles[:, 0:4] = host_tiles[:, 0:4]
         tiles[:, 4] = first
         tiles[:, 5] = per_tile
-        return parts[np.argsort(-(cost / n)[tile], kind="stable")], tiles
+        # parts of a tile with at most four or eight rows go to a kernel for so many, behind
+        # the others
+        rows = [4 if r <= 4 else 8 if r <= 8 else AP_TI for r in host_tiles[:, 1].tolist()]
+        first_cost = -(cost / n)
+        groups = []
+        for r in sorted(set(rows), reverse=True):
+            count = int(per_tile[np.equal(rows, r)].sum())
+            groups.append((sum(g[1] for g in groups), count, r))
+        order = np.argsort(first_cost[tile], kind="stable") if len(groups) == 1 else \
+            np.lexsort((first_cost[tile], -np.asarray(rows)[tile]))
+        return parts[order], tiles, groups
 
     def plan_triangle(self, ids: Optional[Sequence[int]] = None, ldc: Optional[int] = None) -> PairPlan:
         """All pairs i < j among ``ids`` (default: every vector of the arena), and
@@ -823,13 +835,17 @@ class PairEngine:
                 int(plan.mirror)))
         else:
             launch = self.L.phyloPairsLaunchParts if parts else self.L.phyloPairsLaunch
-            check(launch(
-                st, _p(a.pair_keys()), _p(a.values), _p(a.vec_off), _p(a.roff),
-                _p(ca.pair_keys()), _p(ca.values), _p(ca.vec_off), _p(ca.roff), a.R,
-                self.cfg.wshift, _p(plan.rowids), _p(plan.colids),
-                _p(plan.parts if parts else plan.items), plan.nparts if parts else plan.nitems,
-                _p(self.counter), _p(part), self.cfg.fold, cyc, self.cfg.tile_rows,
-                self.cfg.tile_cols, self.grid))
+            items, size = (plan.parts, 48) if parts else (plan.items, 32)
+            groups = plan.part_groups if parts else []
+            groups = groups or [(0, plan.nparts if parts else plan.nitems, self.cfg.tile_rows)]
+            for g, (first, count, rows) in enumerate(groups):
+                check(launch(
+                    st, _p(a.pair_keys()), _p(a.values), _p(a.vec_off), _p(a.roff),
+                    _p(ca.pair_keys()), _p(ca.values), _p(ca.vec_off), _p(ca.roff), a.R,
+                    self.cfg.wshift, _p(plan.rowids), _p(plan.colids), _p(items) + first * size,
+                    count, _p(self.counter) + 4 * g, _p(part), self.cfg.fold, cyc, rows,
+                    self.cfg.tile_cols, self.grid))
+            self.launches += len(groups) - 1
             if events is not None:
                 events[1].record(s_obj)
             upper = (2 if plan.diag and diagonal else 1) if plan.upper else 0

@@ -96,3 +96,30 @@ def test_reduction_sums_every_partial(tj, words, S):
     for t in range(2):
         want[16 * t:32 - (t if t else 16), 5:5 + ncol] = sums[t, :16 - t, :ncol]
     assert torch.equal(out, want)
+
+
+# Row vectors by fours, eights and sixteens: the same sums, bit for bit, whichever kernel
+# takes a part (each row's products enter its own accumulators in the same order).
+@pytest.mark.parametrize("rows", [1, 4, 5, 8, 9, 16, 17, 20, 24, 25])
+@pytest.mark.parametrize("cols,tile_cols", [(3, 128), (37, 128), (50, 256)])
+def test_few_rows(rows, cols, tile_cols):
+    db = _arena("protein", 5, cols, 0.2)
+    queries = _arena("protein", 5, rows, 0.05)
+    cfg = EngineConfig(segments=2, compress=False, tile_cols=tile_cols)
+    PairEngine(db, cfg).ensure_index()
+    eng = PairEngine(queries, cfg)
+    eng.ensure_index()
+    plan = eng.plan_rect(np.arange(rows), np.arange(cols), ldc=cols, col_arena=db)
+    assert plan.host_parts is not None
+    last = rows % 16 or 16
+    small = [4] if last <= 4 else [8] if last <= 8 else [16]
+    assert [g[2] for g in plan.part_groups] == ([16] if rows > 16 and small != [16] else []) + small
+    assert sum(g[1] for g in plan.part_groups) == len(plan.host_parts)
+    outs = []
+    for groups in (plan.part_groups, [(0, len(plan.host_parts), 16)]):
+        plan.part_groups = groups
+        out = torch.full((rows, cols), np.nan, dtype=torch.float64, device="cuda")
+        eng.run(plan, out, diagonal=False, col_arena=db)
+        outs.append(out.cpu().numpy())
+    assert np.array_equal(outs[0], outs[1])
+    assert np.isfinite(outs[0]).all()
