@@ -724,8 +724,15 @@ class PairEngine:
         least = nnz_of_col[host_tiles[:, 2] + ncol - 1] / R
         tail = self.cfg.fold * -(-512 // ncol) / np.maximum(least, 1e-9)
         if fixed:  # as the columns ask, so a pair's arithmetic does not depend on the rows
-            n = np.minimum(math.ceil(windows / PART_WINDOWS), windows / np.maximum(4.0 * tail, 1.0))
-            n = np.maximum(n, 1).astype(np.int64)
+            most = math.ceil(windows / PART_WINDOWS)
+            n = np.maximum(np.minimum(most, windows / np.maximum(4.0 * tail, 1.0)), 1).astype(np.int64)
+            # where that leaves CTAs idle, up to one part each, of which the tail may be half
+            # (K = 7, 24 vectors x 40 in 64 + 64 parts: 39.5 ms; in 144 + 144, on 152 SMs,
+            # 21.6; in 160 + 160, two waves, 29.6)
+            busy = S * int(n[host_tiles[:, 0] == host_tiles[0, 0]].sum())
+            if busy < self.grid:
+                limit = np.minimum(most, windows / np.maximum(tail, 1.0)).astype(np.int64)
+                n = np.maximum(np.minimum(n * self.grid // busy, limit), n)
         else:
             n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S, tail, S,
                                self.grid, goal)

@@ -78,3 +78,24 @@ def test_parts_of_fixed_segments_do_not_depend_on_the_rows():
         cuts.append({tuple(int(x) for x in p[[2, 3, 4, 5, 8, 9]]) for p in first})
     assert cuts[0] == cuts[1]
     assert max(b - a for _, _, a, b, _, _ in cuts[0]) <= engine.PART_WINDOWS
+
+
+@pytest.mark.parametrize("cols,nnz", [(40, 2 * 10 ** 5), (20, 10 ** 5), (5, 10 ** 6), (150, 10 ** 5)])
+def test_small_databases_use_the_idle_ctas(cols, nnz):
+    """Few columns of few entries: more parts than their tails alone would ask for, at most
+    one per CTA, and the same whatever the rows."""
+    grid, cuts = 152, []
+    for rows in (np.arange(3), np.arange(40)):
+        eng = _engine(np.full(200, nnz), 41878, grid=grid, segments=16)
+        plan = eng.plan_rect(rows, np.arange(cols), ldc=cols, col_arena=eng.arena)
+        _check(plan)
+        first = plan.host_parts[(plan.host_parts[:, 0] == 0)]
+        # parts whose tails are a quarter of them at most, as many as there are
+        free = 0
+        for c0, ncol in {(int(p[2]), int(p[3])) for p in first}:
+            tail = eng.cfg.fold * -(-512 // ncol) / (nnz / 41878)
+            windows = 41878 / 16
+            free += 16 * max(1, int(min(-(-windows // engine.PART_WINDOWS), windows / max(4 * tail, 1))))
+        assert free <= len(first) <= max(grid, free)
+        cuts.append({tuple(int(x) for x in p[[2, 3, 4, 5, 8, 9]]) for p in first})
+    assert cuts[0] == cuts[1]
