@@ -218,8 +218,11 @@ __device__ __forceinline__ uint64_t c1_index(const BuildArgs &a, int p, uint32_t
     return (uint64_t)t.x + (uint32_t)__popc(t.y & ((1u << (q & 31u)) - 1u));
 }
 
+// Count at index i of them; 0 past the entries there is room for, which only a build out of
+// candidate room asks for (its alphas are discarded).
 __device__ __forceinline__ uint32_t c1_load(const BuildArgs &a, uint64_t i) {
-    return a.compact1 ? __ldg(&a.cc[i].x) : __ldg(&a.c1[i]);
+    if (!a.compact1) return __ldg(&a.c1[i]);
+    return i < a.cap1 ? __ldg(&a.cc[i].x) : 0u;
 }
 
 // Index of (K-2)-mer m of proteome p in c2: dense row entry, or its rank among
