@@ -190,8 +190,9 @@ int phyloWindowIndex(uintptr_t stream, uintptr_t d_keys, uintptr_t d_vec_off, in
  * vector, windows up to 2^10 keys.  Partial blocks are tile_rows x tile_cols
  * float pairs. */
 
-/* Sets the pair kernel's shared-memory limit for this window width and
- * reports how many CTAs fit on one SM. */
+/* Sets the pair kernel's shared-memory limit (that of the widest window, so one
+ * caller's window does not narrow another's) and reports how many CTAs fit on one
+ * SM with this window width. */
 int phyloPairsPrepare(int window_shift, int tile_rows, int tile_cols, int *ctas_per_sm);
 
 /* Dynamic shared memory of the pair kernel; -1 for an unknown tile shape. */

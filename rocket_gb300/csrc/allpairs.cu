@@ -769,12 +769,16 @@ static size_t ap_parts_smem(uint32_t wshift, int rows) {
 cudaError_t ap_prepare(uint32_t wshift, int tile_rows, int tile_cols, int *ctas_per_sm) {
     const size_t smem = ap_smem_bytes(wshift, tile_rows, tile_cols);
     const void *fn = ap_kernel(wshift, tile_rows, tile_cols);
-    PHYLO_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The limit is the kernel's, whoever asked for it, so it is that of the widest window:
+    // the caller's own would take the launches from callers with wider ones.
+    const uint32_t widest = (uint32_t)ap_max_wshift(tile_rows, tile_cols);
+    PHYLO_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ap_smem_bytes(widest, tile_rows, tile_cols)));
     if (tile_rows == AP_TI && tile_cols >= 128)
         for (int rows = 4; rows <= AP_TI; rows *= 2)
             PHYLO_CHECK(cudaFuncSetAttribute(ap_parts_kernel(rows, tile_cols),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)ap_parts_smem(wshift, rows)));
+                                             (int)ap_parts_smem(widest, rows)));
     if (ctas_per_sm) {
         int n = 0;
         PHYLO_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
