@@ -333,9 +333,11 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
         uint4 pk[AP_STAGE];
         float4 pv[AP_STAGE];
         auto prefetch_row = [&](uint32_t lo, uint32_t hi) {
+            const uint32_t e0 = 4u * ((lo >> 2) + sl);
+            if (ROWS == 16 && e0 >= hi) return;
 #pragma unroll
             for (uint32_t k = 0; k < AP_STAGE; k++) {
-                const uint32_t e = 4u * ((lo >> 2) + sl + k * SL);
+                const uint32_t e = e0 + 4u * k * SL;
                 if (e < hi) {
                     pk[k] = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
                     pv[k] = __ldg(reinterpret_cast<const float4 *>(rvals + e));
@@ -352,36 +354,45 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
 
         for (uint32_t r = item.w0; r < s1; r++) {
             // scatter window r of row rr: prefetched groups, the rest loaded.  held: window
-            // offsets of the prefetched entries, to clear them (W: none)
+            // offsets of the prefetched entries, to clear them (W: none).  Where windows are
+            // sparse nearly every thread of 16 rows has none and skips all of it: 93 uneven
+            // vectors on their raw K = 7 keys, 2 row entries per window, 48.1 -> 45.3 ms, on
+            // key ranks, 38 per window, 5.33 -> 5.22; 128 uniform proteomes at K = 6, 136 per
+            // window, 6.95 -> 6.93.  (Fewer rows have more threads each: 8 of them 28.0 ->
+            // 29.9 with the branch, K = 7 against 160 vectors.)
             uint32_t held[2 * AP_STAGE];
+            uint32_t rest = 0, rest_hi = 0;
+            const bool scatters = ROWS < 16 || 4u * ((r_lo >> 2) + sl) < r_hi;
+            if (scatters) {
 #pragma unroll
-            for (uint32_t k = 0; k < AP_STAGE; k++) {
-                const uint32_t e = 4u * ((r_lo >> 2) + sl + k * SL);
-                held[2 * k] = held[2 * k + 1] = W | W << 16;
-                if (e < r_hi) {
-                    const uint32_t ks[4] = {pk[k].x, pk[k].y, pk[k].z, pk[k].w};
-                    const float vs[4] = {pv[k].x, pv[k].y, pv[k].z, pv[k].w};
-                    uint32_t off[4];
+                for (uint32_t k = 0; k < AP_STAGE; k++) {
+                    const uint32_t e = 4u * ((r_lo >> 2) + sl + k * SL);
+                    held[2 * k] = held[2 * k + 1] = W | W << 16;
+                    if (e < r_hi) {
+                        const uint32_t ks[4] = {pk[k].x, pk[k].y, pk[k].z, pk[k].w};
+                        const float vs[4] = {pv[k].x, pv[k].y, pv[k].z, pv[k].w};
+                        uint32_t off[4];
 #pragma unroll
-                    for (uint32_t u = 0; u < 4; u++) {
-                        const bool in = e + u >= r_lo && e + u < r_hi;
-                        off[u] = in ? ks[u] & wmask : W;
-                        if (in) drow[off[u] * ROWS] = vs[u];
+                        for (uint32_t u = 0; u < 4; u++) {
+                            const bool in = e + u >= r_lo && e + u < r_hi;
+                            off[u] = in ? ks[u] & wmask : W;
+                            if (in) drow[off[u] * ROWS] = vs[u];
+                        }
+                        held[2 * k] = off[0] | off[1] << 16;
+                        held[2 * k + 1] = off[2] | off[3] << 16;
                     }
-                    held[2 * k] = off[0] | off[1] << 16;
-                    held[2 * k + 1] = off[2] | off[3] << 16;
                 }
-            }
-            const uint32_t rest = 4u * ((r_lo >> 2) + sl + AP_STAGE * SL);
-            const uint32_t rest_hi = r_hi;
-            for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
-                const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
-                const float4 vv = __ldg(reinterpret_cast<const float4 *>(rvals + e));
-                const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
-                const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
+                rest = 4u * ((r_lo >> 2) + sl + AP_STAGE * SL);
+                rest_hi = r_hi;
+                for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
+                    const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
+                    const float4 vv = __ldg(reinterpret_cast<const float4 *>(rvals + e));
+                    const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
+                    const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
 #pragma unroll
-                for (uint32_t u = 0; u < 4; u++)
-                    if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = vs[u];
+                    for (uint32_t u = 0; u < 4; u++)
+                        if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = vs[u];
+                }
             }
             // the next window's row entries
             r_lo = r_hi;
@@ -444,17 +455,19 @@ __global__ void __launch_bounds__(THREADS, MINB) k_allpairs(ApArgs a) {
             else  // a lane inside a run with entries of the segment left
                 more = __syncthreads_or(nacc > 0 && cur != AP_DONE && c_lo < c_end);
             // clear window r of row rr
+            if (scatters) {
 #pragma unroll
-            for (uint32_t k = 0; k < 2 * AP_STAGE; k++) {
-                if ((held[k] & 0xffffu) != W) drow[(held[k] & 0xffffu) * ROWS] = 0.0f;
-                if (held[k] >> 16 != W) drow[(held[k] >> 16) * ROWS] = 0.0f;
-            }
-            for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
-                const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
-                const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
+                for (uint32_t k = 0; k < 2 * AP_STAGE; k++) {
+                    if ((held[k] & 0xffffu) != W) drow[(held[k] & 0xffffu) * ROWS] = 0.0f;
+                    if (held[k] >> 16 != W) drow[(held[k] >> 16) * ROWS] = 0.0f;
+                }
+                for (uint32_t e = rest; e < rest_hi; e += 4u * SL) {
+                    const uint4 kk = __ldg(reinterpret_cast<const uint4 *>(rkeys + e));
+                    const uint32_t ks[4] = {kk.x, kk.y, kk.z, kk.w};
 #pragma unroll
-                for (uint32_t u = 0; u < 4; u++)
-                    if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = 0.0f;
+                    for (uint32_t u = 0; u < 4; u++)
+                        if (e + u < rest_hi) drow[(ks[u] & wmask) * ROWS] = 0.0f;
+                }
             }
             if (PARTS && !more) break;
             bar_sync(1 + (int)wg, 128);
