@@ -38,6 +38,9 @@ AP_TJ = 128         # default column vectors per work item (512-thread CTAs)
 PART_WINDOWS = 128  # windows per part of a segment fixed by EngineConfig.segments, at most
                     # (24 queries x 160 vectors in 16 segments: 14.6 ms; 15.2 / 15.8 / 18.9
                     # with 64 / 256 / 512)
+PARTS_PER_CTA = 4.5  # parts per CTA of one row tile's fixed segments, at most (rounded up for
+                     # every tile)
+WINDOW_ENTRIES = 4e4  # cost of a window, in column entries, by which they are shared out
 PART_SETUP = 2.0    # cost of starting and ending an item, in windows
 NSYM = {"protein": 21, "DNA": 4}
 
@@ -62,6 +65,42 @@ def auto_tile_cols(n_cols: int) -> int:
     full; in a triangle over fewer than 384 vectors most 256-column items would be
     half empty, and 128-column items keep more lanes busy."""
     return 256 if n_cols >= 384 else 128
+
+
+def part_tails(fold: int, ncol: np.ndarray, least: np.ndarray) -> np.ndarray:
+    """Windows a part of a segment goes on past its own, until each of its lanes has
+    finished the FP32 run it is in: those in which the sparsest of the tile's ``ncol``
+    columns, of ``least`` entries per window, has a run's entries per lane."""
+    return fold * -(-512 // np.maximum(ncol, 1)) / np.maximum(least, 1e-9)
+
+
+def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray,
+                nnz: np.ndarray, entries: np.ndarray, first=slice(None)) -> np.ndarray:
+    """Parts per segment of each tile of a plan of ``S`` fixed segments over ``R`` windows,
+    from what the columns alone say (``ncol`` of each tile, ``nnz`` of its sparsest,
+    ``entries`` of all of them), so that a pair's arithmetic does not depend on the rows it
+    runs with.  ``first``: the tiles of the first row tile, all that a plan of few rows has."""
+    windows = R / S
+    tail = part_tails(cfg.fold, ncol, nnz / R)
+    most = math.ceil(windows / PART_WINDOWS)
+    n = np.maximum(np.minimum(most, windows / np.maximum(4.0 * tail, 1.0)), 1).astype(np.int64)
+    # where that leaves CTAs idle, up to one part each, of which the tail may be half
+    # (K = 7, 24 vectors x 40 in 64 + 64 parts: 39.5 ms; in 144 + 144, on 152 SMs,
+    # 21.6; in 160 + 160, two waves, 29.6)
+    busy = S * int(n[first].sum())
+    if busy < grid:
+        limit = np.minimum(most, windows / np.maximum(tail, 1.0)).astype(np.int64)
+        n = np.maximum(np.minimum(n * grid // busy, limit), n)
+    # no more than the columns need to fill the GPU, in proportion to the tiles' work.  Every
+    # part costs a tail and a count of what comes before it, and a partial block: 64 uneven
+    # vectors against 2,048 in 16 segments, K = 7, took 2,914 ms in 170,000 parts, 635 in 3,072
+    # (587 before there were parts), one vector 648, 96 and 158; K = 6 224, 208 and 240, one
+    # vector 32.2, 29.7 and 133.  Shared out by entries alone (WINDOW_ENTRIES 2,000) the
+    # windows of sparse tiles are waited for: K = 6, 8 against 512 12.1 ms, 10.8 with 10,000.
+    work = entries + WINDOW_ENTRIES * R
+    share = PARTS_PER_CTA * grid / S * work / work[first].sum()
+    n = np.minimum(n, np.ceil(share).astype(np.int64))
+    return n
 
 
 def split_segments(windows: np.ndarray, cost: np.ndarray, tail: np.ndarray, count: int,
@@ -718,25 +757,19 @@ class PairEngine:
         if ntiles == 0 or (not fixed and ntiles * S >= goal):
             return None
         ncol = np.maximum(host_tiles[:, 3], 1)
-        windows = R / S
-        # a part goes on past its own windows until each of its lanes has finished the FP32
-        # run it is in: the windows in which the tile's sparsest column has one per lane
-        least = nnz_of_col[host_tiles[:, 2] + ncol - 1] / R
-        tail = self.cfg.fold * -(-512 // ncol) / np.maximum(least, 1e-9)
-        if fixed:  # as the columns ask, so a pair's arithmetic does not depend on the rows
-            most = math.ceil(windows / PART_WINDOWS)
-            n = np.maximum(np.minimum(most, windows / np.maximum(4.0 * tail, 1.0)), 1).astype(np.int64)
-            # where that leaves CTAs idle, up to one part each, of which the tail may be half
-            # (K = 7, 24 vectors x 40 in 64 + 64 parts: 39.5 ms; in 144 + 144, on 152 SMs,
-            # 21.6; in 160 + 160, two waves, 29.6)
-            busy = S * int(n[host_tiles[:, 0] == host_tiles[0, 0]].sum())
-            if busy < self.grid:
-                limit = np.minimum(most, windows / np.maximum(tail, 1.0)).astype(np.int64)
-                n = np.maximum(np.minimum(n * self.grid // busy, limit), n)
+        least = nnz_of_col[host_tiles[:, 2] + ncol - 1]
+        if fixed:
+            ends = np.concatenate([[0], np.cumsum(nnz_of_col)])
+            entries = ends[host_tiles[:, 2] + host_tiles[:, 3]] - ends[host_tiles[:, 2]]
+            n = fixed_parts(self.cfg, R, self.grid, S, ncol, least, entries,
+                            host_tiles[:, 0] == host_tiles[0, 0])
         else:
-            n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S, tail, S,
-                               self.grid, goal)
-        if n.max() == 1:
+            n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S,
+                               part_tails(self.cfg.fold, ncol, least / R), S, self.grid, goal)
+        # one part each: whole items, unless an eighth of the tiles are of few rows, which have
+        # kernels of their own (11,000 vectors of 200 proteins, K = 6, against 1 row 39.3 ->
+        # 23.4 ms, 24 rows 79.6 -> 73.4; the 16-row kernel of parts takes 4 to 7% longer)
+        if n.max() == 1 and not (fixed and (host_tiles[:, 1] <= 8).mean() >= 0.125):
             return None
         per_tile = n * S
         tile = np.repeat(np.arange(ntiles), per_tile)
