@@ -103,6 +103,25 @@ def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray
     return n
 
 
+def fixed_blocks(cfg: "EngineConfig", R: int, grid: int, rows: int, nnz: np.ndarray) -> int:
+    """Partial blocks of a plan of fixed segments (EngineConfig.segments) for ``rows`` vectors
+    against columns of ``nnz`` entries: what PairEngine.plan_rect makes of them."""
+    S = min(cfg.segments, max(1, R))
+    nnz = -np.sort(-np.asarray(nnz, np.int64))
+    col0 = np.arange(0, max(len(nnz), 1), cfg.tile_cols)
+    per_segment = len(col0)
+    if len(nnz) and can_cut(cfg):
+        end = np.minimum(col0 + cfg.tile_cols, len(nnz))
+        per_segment = int(fixed_parts(cfg, R, grid, S, end - col0, nnz[end - 1],
+                                      np.add.reduceat(nnz, col0)).sum())
+    return -(-rows // cfg.tile_rows) * S * per_segment
+
+
+def can_cut(cfg: "EngineConfig") -> bool:
+    """Whether the pair kernel of the configuration's tiles runs parts of segments."""
+    return cfg.algorithm == "window" and cfg.tile_rows == AP_TI and cfg.tile_cols >= 128
+
+
 def split_segments(windows: np.ndarray, cost: np.ndarray, tail: np.ndarray, count: int,
                    grid: int, most: int) -> np.ndarray:
     """Parts per segment of a window plan with too few segments to fill the GPU.  A part
@@ -719,8 +738,7 @@ class PairEngine:
         dev = self.device
         parts = part_tiles = np.zeros((0, 0), np.int64)
         cut = None
-        if self.cfg.algorithm == "window" and self.cfg.tile_rows == AP_TI and \
-                self.cfg.tile_cols >= 128:
+        if can_cut(self.cfg):
             cut = self._cut_items(S, cost, host_tiles, col_nnz[colids])
             if cut is not None:
                 parts, part_tiles, groups = cut

@@ -29,7 +29,6 @@ from __future__ import annotations
 
 import collections
 import dataclasses
-import math
 import threading
 import time
 from dataclasses import dataclass, field
@@ -39,8 +38,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .engine import (PART_WINDOWS, Arena, BatchBuilder, EngineConfig, PairEngine,
-                     key_limit)
+from .engine import Arena, BatchBuilder, EngineConfig, PairEngine, fixed_blocks, key_limit
 from .synth import Proteomes
 
 
@@ -197,6 +195,7 @@ class ServingEngine:
         self.threads: List[threading.Thread] = []
         self.slots: List[_Slot] = []
         self.tuned: Optional[dict] = None
+        self.grid = 1  # CTAs of the pair kernel, once a database is loaded
 
     # -- database -----------------------------------------------------------
     def load(self, proteomes: Proteomes, capacity_vectors: Optional[int] = None,
@@ -216,6 +215,7 @@ class ServingEngine:
         # build into a staging arena of exactly the database's capacity class
         built = builder.build(seq, proteomes.offsets, stream=stream)
         eng = PairEngine(built, self.cfg)
+        self.grid = eng.grid
         eng.ensure_index(stream)
         if not db.append(built, stream):
             raise MemoryError("database does not fit its capacity")
@@ -236,7 +236,7 @@ class ServingEngine:
         n = db.n
         row_ids = np.arange(min(rows, n))
         out = torch.empty((len(row_ids), n), dtype=torch.float64, device=self.device)
-        results = []
+        results, grids = [], {}
         for w in widths:
             cfg = dataclasses.replace(self.cfg, tile_cols=int(w))
             eng = PairEngine(db, cfg)
@@ -253,7 +253,9 @@ class ServingEngine:
                 torch.cuda.synchronize(self.device)
                 best = min(best, e0.elapsed_time(e1))
             results.append({"tile_cols": int(w), "ms": best})
+            grids[int(w)] = eng.grid
         win = min(results, key=lambda r: r["ms"])
+        self.grid = grids[win["tile_cols"]]
         self.cfg = dataclasses.replace(self.cfg, tile_cols=win["tile_cols"])
         self.tuned = dict(win, rows=len(row_ids), db=n, candidates=results)
         return self.tuned
@@ -294,12 +296,8 @@ class ServingEngine:
                                                  min(nq, self.max_batch), int(cand)))
         staged = float(np.sum(8 * lens + 64)) * 8.0
         roff = nq * (self.db.R + 1) * 4.0
-        ti = self.cfg.tile_rows
-        tj = self.cfg.tile_cols
-        tiles = math.ceil(nq / ti) * math.ceil(max(db_n, 1) / tj)
-        # a segment's items may run in parts, each with a partial block of its own
-        per_segment = math.ceil(math.ceil(self.db.R / self.cfg.segments) / PART_WINDOWS)
-        parts = tiles * self.cfg.segments * per_segment * ti * tj * 8.0
+        blocks = fixed_blocks(self.cfg, self.db.R, self.grid, nq, self.db.arena.nnz[:db_n])
+        parts = blocks * self.cfg.tile_rows * self.cfg.tile_cols * 8.0
         out = nq * max(db_n, 1) * 8.0
         return scratch + staged + roff + parts + out
 
