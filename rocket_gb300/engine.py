@@ -75,11 +75,11 @@ def part_tails(fold: int, ncol: np.ndarray, least: np.ndarray) -> np.ndarray:
 
 
 def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray,
-                nnz: np.ndarray, entries: np.ndarray, first=slice(None)) -> np.ndarray:
+                nnz: np.ndarray, entries: np.ndarray, alone=slice(None)) -> np.ndarray:
     """Parts per segment of each tile of a plan of ``S`` fixed segments over ``R`` windows,
     from what the columns alone say (``ncol`` of each tile, ``nnz`` of its sparsest,
     ``entries`` of all of them), so that a pair's arithmetic does not depend on the rows it
-    runs with.  ``first``: the tiles of the first row tile, all that a plan of few rows has."""
+    runs with.  ``alone``: the tiles that have to fill the GPU, of one row tile of a query."""
     windows = R / S
     tail = part_tails(cfg.fold, ncol, nnz / R)
     most = math.ceil(windows / PART_WINDOWS)
@@ -87,7 +87,7 @@ def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray
     # where that leaves CTAs idle, up to one part each, of which the tail may be half
     # (K = 7, 24 vectors x 40 in 64 + 64 parts: 39.5 ms; in 144 + 144, on 152 SMs,
     # 21.6; in 160 + 160, two waves, 29.6)
-    busy = S * int(n[first].sum())
+    busy = S * int(n[alone].sum())
     if busy < grid:
         limit = np.minimum(most, windows / np.maximum(tail, 1.0)).astype(np.int64)
         n = np.maximum(np.minimum(n * grid // busy, limit), n)
@@ -98,7 +98,7 @@ def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray
     # vector 32.2, 29.7 and 133.  Shared out by entries alone (WINDOW_ENTRIES 2,000) the
     # windows of sparse tiles are waited for: K = 6, 8 against 512 12.1 ms, 10.8 with 10,000.
     work = entries + WINDOW_ENTRIES * R
-    share = PARTS_PER_CTA * grid / S * work / work[first].sum()
+    share = PARTS_PER_CTA * grid / S * work / work[alone].sum()
     n = np.minimum(n, np.ceil(share).astype(np.int64))
     return n
 
@@ -739,7 +739,7 @@ class PairEngine:
         parts = part_tiles = np.zeros((0, 0), np.int64)
         cut = None
         if can_cut(self.cfg):
-            cut = self._cut_items(S, cost, host_tiles, col_nnz[colids])
+            cut = self._cut_items(S, cost, host_tiles, col_nnz[colids], upper)
             if cut is not None:
                 parts, part_tiles, groups = cut
                 nparts = len(parts)
@@ -764,7 +764,7 @@ class PairEngine:
             plan.part_groups = groups
         return plan
 
-    def _cut_items(self, S, cost, host_tiles, nnz_of_col):
+    def _cut_items(self, S, cost, host_tiles, nnz_of_col, upper):
         """(parts [n, 12], tiles [ntiles, 8], launches) of a plan of S segments per tile whose items
         are too few to fill the GPU, longest first, or None where no segment is cut.
         ``cost``: of each tile; ``nnz_of_col``: entries of the plan's columns in their
@@ -776,11 +776,12 @@ class PairEngine:
             return None
         ncol = np.maximum(host_tiles[:, 3], 1)
         least = nnz_of_col[host_tiles[:, 2] + ncol - 1]
+        ends = np.concatenate([[0], np.cumsum(nnz_of_col)])
+        entries = ends[host_tiles[:, 2] + host_tiles[:, 3]] - ends[host_tiles[:, 2]]
         if fixed:
-            ends = np.concatenate([[0], np.cumsum(nnz_of_col)])
-            entries = ends[host_tiles[:, 2] + host_tiles[:, 3]] - ends[host_tiles[:, 2]]
-            n = fixed_parts(self.cfg, R, self.grid, S, ncol, least, entries,
-                            host_tiles[:, 0] == host_tiles[0, 0])
+            # (a triangle's tiles run together; a query's first row tile may be all it has)
+            alone = slice(None) if upper else host_tiles[:, 0] == host_tiles[0, 0]
+            n = fixed_parts(self.cfg, R, self.grid, S, ncol, least, entries, alone)
         else:
             n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S,
                                part_tails(self.cfg.fold, ncol, least / R), S, self.grid, goal)
@@ -810,15 +811,21 @@ class PairEngine:
         tiles[:, 4] = first
         tiles[:, 5] = per_tile
         # parts of a tile with at most four or eight rows go to a kernel for so many, behind
-        # the others
-        rows = [4 if r <= 4 else 8 if r <= 8 else AP_TI for r in host_tiles[:, 1].tolist()]
-        first_cost = -(cost / n)
-        groups = []
-        for r in sorted(set(rows), reverse=True):
-            count = int(per_tile[np.equal(rows, r)].sum())
-            groups.append((sum(g[1] for g in groups), count, r))
-        order = np.argsort(first_cost[tile], kind="stable") if len(groups) == 1 else \
-            np.lexsort((first_cost[tile], -np.asarray(rows)[tile]))
+        # the others; in a triangle of fixed segments, where only the last tiles are of so few and
+        # their items as long as any, not where a launch of their own would leave half of the
+        # CTAs idle (16 segments, K = 6, 200 vectors of 300 proteins: 3.30 -> 2.91 ms, 2.87
+        # uncut; K = 7, 200 uneven 28.5 -> 25.8)
+        rows = np.where(host_tiles[:, 1] <= 4, 4, np.where(host_tiles[:, 1] <= 8, 8, AP_TI))
+        for few in (4, 8):
+            mine, more = rows == few, rows > few
+            if fixed and upper and more.any() and 2 * per_tile[mine].sum() < self.grid:
+                rows[mine] = rows[more].min()
+        groups, at = [], 0
+        for r in sorted(set(rows.tolist()), reverse=True):
+            count = int(per_tile[rows == r].sum())
+            groups.append((at, count, r))
+            at += count
+        order = np.lexsort((-(cost / n)[tile], -rows[tile]))
         return parts[order], tiles, groups
 
     def plan_triangle(self, ids: Optional[Sequence[int]] = None, ldc: Optional[int] = None) -> PairPlan:

@@ -61,3 +61,20 @@ def test_whole_segments_of_few_rows_keep_their_kernels():
     assert plan.nparts == plan.nitems and [g[2] for g in plan.part_groups] == [8]
     assert (plan.host_parts[:, 4:6] == plan.host_parts[:, 8:10]).all()
     assert _plan(nnz, 41878, 48, 20000).host_parts is None
+
+
+@pytest.mark.parametrize("n,R", [(40, 3000), (200, 41878), (200, 8000), (24, 224), (500, 41878)])
+@pytest.mark.parametrize("segments", [2, 16, 64])
+def test_triangles_fill_the_gpu_together(n, R, segments):
+    """All tiles of a triangle share the GPU: its fixed segments take no more parts than fill
+    it, and the last rows' tiles a launch of their own only where they fill half of it."""
+    eng = _engine(np.full(n, 200 * R), R, grid=GRID, segments=segments)
+    plan = eng.plan_triangle()
+    if plan.host_parts is None:
+        return
+    _check(plan)
+    assert plan.nparts <= engine.PARTS_PER_CTA * GRID + plan.S * plan.ntiles
+    assert sum(g[1] for g in plan.part_groups) == plan.nparts
+    for first, count, rows in plan.part_groups:
+        assert (plan.host_parts[first:first + count, 1] <= rows).all()
+        assert rows == 16 or 2 * count >= GRID
