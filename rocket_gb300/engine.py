@@ -97,9 +97,10 @@ def fixed_parts(cfg: "EngineConfig", R: int, grid: int, S: int, ncol: np.ndarray
     # (587 before there were parts), one vector 648, 96 and 158; K = 6 224, 208 and 240, one
     # vector 32.2, 29.7 and 133.  Shared out by entries alone (WINDOW_ENTRIES 2,000) the
     # windows of sparse tiles are waited for: K = 6, 8 against 512 12.1 ms, 10.8 with 10,000.
-    work = entries + WINDOW_ENTRIES * R
-    share = PARTS_PER_CTA * grid / S * work / work[alone].sum()
-    n = np.minimum(n, np.ceil(share).astype(np.int64))
+    room = PARTS_PER_CTA * grid / S
+    if n[alone].sum() > room:
+        work = entries + WINDOW_ENTRIES * R
+        n = np.minimum(n, np.ceil(room / work[alone].sum() * work).astype(np.int64))
     return n
 
 
@@ -776,19 +777,21 @@ class PairEngine:
             return None
         ncol = np.maximum(host_tiles[:, 3], 1)
         least = nnz_of_col[host_tiles[:, 2] + ncol - 1]
-        ends = np.concatenate([[0], np.cumsum(nnz_of_col)])
-        entries = ends[host_tiles[:, 2] + host_tiles[:, 3]] - ends[host_tiles[:, 2]]
         if fixed:
+            ends = np.concatenate([[0], np.cumsum(nnz_of_col)])
+            entries = ends[host_tiles[:, 2] + host_tiles[:, 3]] - ends[host_tiles[:, 2]]
             # (a triangle's tiles run together; a query's first row tile may be all it has)
             alone = slice(None) if upper else host_tiles[:, 0] == host_tiles[0, 0]
             n = fixed_parts(self.cfg, R, self.grid, S, ncol, least, entries, alone)
         else:
             n = split_segments(np.full(ntiles, float(max(R // S, 1))), cost / S,
                                part_tails(self.cfg.fold, ncol, least / R), S, self.grid, goal)
-        # one part each: whole items, unless an eighth of the tiles are of few rows, which have
-        # kernels of their own (11,000 vectors of 200 proteins, K = 6, against 1 row 39.3 ->
-        # 23.4 ms, 24 rows 79.6 -> 73.4; the 16-row kernel of parts takes 4 to 7% longer)
-        if n.max() == 1 and not (fixed and (host_tiles[:, 1] <= 8).mean() >= 0.125):
+        # one part each: whole items, unless the columns fill the GPU so and an eighth of the
+        # tiles are of few rows, which have kernels of their own (11,000 vectors of 200 proteins,
+        # K = 6, against 1 row 39.3 -> 23.4 ms, 24 rows 79.6 -> 73.4; the 16-row kernel of parts
+        # takes 4 to 7% longer)
+        if n.max() == 1 and not (fixed and not upper and S * np.count_nonzero(alone) >= self.grid
+                                 and (host_tiles[:, 1] <= 8).mean() >= 0.125):
             return None
         per_tile = n * S
         tile = np.repeat(np.arange(ntiles), per_tile)
@@ -815,17 +818,21 @@ class PairEngine:
         # their items as long as any, not where a launch of their own would leave half of the
         # CTAs idle (16 segments, K = 6, 200 vectors of 300 proteins: 3.30 -> 2.91 ms, 2.87
         # uncut; K = 7, 200 uneven 28.5 -> 25.8)
-        rows = np.where(host_tiles[:, 1] <= 4, 4, np.where(host_tiles[:, 1] <= 8, 8, AP_TI))
-        for few in (4, 8):
-            mine, more = rows == few, rows > few
-            if fixed and upper and more.any() and 2 * per_tile[mine].sum() < self.grid:
-                rows[mine] = rows[more].min()
+        rows = [4 if r <= 4 else 8 if r <= 8 else AP_TI for r in host_tiles[:, 1].tolist()]
+        for few in (4, 8) if fixed and upper else ():
+            mine, more = np.equal(rows, few), [r for r in rows if r > few]
+            if more and 2 * per_tile[mine].sum() < self.grid:
+                rows = np.where(mine, min(more), rows).tolist()
+        kinds = sorted(set(rows), reverse=True)
+        first_cost = -(cost / n)
+        if len(kinds) == 1:
+            return parts[np.argsort(first_cost[tile], kind="stable")], tiles, [(0, len(tile), kinds[0])]
         groups, at = [], 0
-        for r in sorted(set(rows.tolist()), reverse=True):
-            count = int(per_tile[rows == r].sum())
+        for r in kinds:
+            count = int(per_tile[np.equal(rows, r)].sum())
             groups.append((at, count, r))
             at += count
-        order = np.lexsort((-(cost / n)[tile], -rows[tile]))
+        order = np.lexsort((first_cost[tile], -np.asarray(rows)[tile]))
         return parts[order], tiles, groups
 
     def plan_triangle(self, ids: Optional[Sequence[int]] = None, ldc: Optional[int] = None) -> PairPlan:
