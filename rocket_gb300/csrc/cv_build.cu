@@ -218,11 +218,8 @@ __device__ __forceinline__ uint64_t c1_index(const BuildArgs &a, int p, uint32_t
     return (uint64_t)t.x + (uint32_t)__popc(t.y & ((1u << (q & 31u)) - 1u));
 }
 
-// Count at index i of them; 0 past the entries there is room for, which only a build out of
-// candidate room asks for (its alphas are discarded).
 __device__ __forceinline__ uint32_t c1_load(const BuildArgs &a, uint64_t i) {
-    if (!a.compact1) return __ldg(&a.c1[i]);
-    return i < a.cap1 ? __ldg(&a.cc[i].x) : 0u;
+    return a.compact1 ? __ldg(&a.cc[i].x) : __ldg(&a.c1[i]);
 }
 
 // Index of (K-2)-mer m of proteome p in c2: dense row entry, or its rank among
@@ -827,6 +824,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 6) k_alpha(BuildArgs a) {
     const uint64_t seg = c * (ALPHA_TILE / SEG) + w;
     const uint64_t total = min(*a.cand_total, a.cand_cap);
     if (g0 >= total) return;  // past the last proteome: k_norm and k_compact stop there too
+    // out of room: the ranks below may lie past the count tables, and nothing is kept
+    if (*a.status) return;
     const int p = find_owner(a.cbase, a.B, g0);
     const uint32_t np =
         (uint32_t)(a.chunk_cand_off[(uint64_t)(p + 1) * a.NCH] - a.chunk_cand_off[(uint64_t)p * a.NCH]);
@@ -957,7 +956,8 @@ __global__ void __launch_bounds__(NORM_THREADS) k_norm(BuildArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t ncta = a.cand_cap / ALPHA_TILE;
     const uint64_t c0 = min(a.cbase[p] / ALPHA_TILE, ncta);
-    const uint64_t c1 = min(a.cbase[p + 1] / ALPHA_TILE, ncta);
+    // out of room, k_alpha left no partials: no entries
+    const uint64_t c1 = *a.status ? c0 : min(a.cbase[p + 1] / ALPHA_TILE, ncta);
     U192 acc = {0, 0, 0};
     uint64_t m1 = 0, run = 0;
     uint32_t bad = 0;
