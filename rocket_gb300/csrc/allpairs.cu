@@ -189,7 +189,7 @@ __device__ __forceinline__ void bar_sync(int id, int n) {
 // the rest of the run begun there, and goes on past its last window until each of its
 // lanes has finished its own run.  The sums are those of the whole segment, bit for bit up
 // to the order of the compensated additions (sums cut anywhere else differ by 1e-9).  24
-// queries against 160 vectors, 64 segments of which the longest took 68 ms: 14.6 ms.
+// queries against 160 vectors, 64 segments of which the longest took 68 ms: 14.4 ms.
 //
 // Visits of a lane (the q-th of its column's L, the segment's first group g0) in the
 // windows [s0, w0): one per group that ends by the first entry of w0 (done), and one per
@@ -743,7 +743,8 @@ static int ap_lpc(int tile_cols) { return tile_cols == 256 ? 2 : AP_LPC; }
 
 size_t ap_smem_bytes(uint32_t wshift, int tile_rows, int tile_cols) {
     if (tile_rows == 32) return r32_smem_bytes(wshift);
-    // (the 64- and 32-column shapes' callers were told 80 bytes per record)
+    // (64- and 32-column shapes: 80 bytes a record as ever, though theirs have 64 too.  The CTAs
+    // per SM, and with them a plan's segments and its sums, follow from this size.)
     return (((size_t)1 << wshift) + 1) * (tile_cols >= 128 ? D_REC : 80u) +
            ap_ring_bytes(tile_cols * ap_lpc(tile_cols));
 }

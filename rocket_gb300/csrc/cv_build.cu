@@ -1231,9 +1231,9 @@ static void build_layout(const BuildGeometry &g, int B, uint64_t cand_cap, Build
     take(r.seen1, nw1);
     take(r.seen2, compact2 ? nw2 : 0);
     if (!compact2) take(r.c2, r.cap2);
-    // at the smallest K the counters are a few hot lines, 4 KB apart as counters side by side
-    // meet in the L2: 12,000 proteins at K = 3 took 1,010 to 1,440 us from one scratch address
-    // to the next, and 1,002 to 1,141 so
+    // At the smallest K these and c1 are a few lines that take every window's atomics, and side
+    // by side they meet in the L2 or not as the scratch's address has it: 12,000 proteins at
+    // K = 3 took 1,012 to 1,448 us over forty addresses, with 4 KB between them 1,002 to 1,141.
     uint32_t *apart = nullptr;
     take(apart, 1024);
     if (!compact) take(r.c1, r.cap1);

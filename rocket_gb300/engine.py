@@ -60,10 +60,13 @@ def key_limit(alphabet: str, k: int) -> int:
 
 def auto_tile_cols(n_cols: int) -> int:
     """Column vectors per work item for plans over ``n_cols`` columns.  Items of 256
-    columns (two lanes per column) spread each window's row scatter and barriers
-    over twice the columns, which pays once the row tiles' column spans are mostly
-    full; in a triangle over fewer than 384 vectors most 256-column items would be
-    half empty, and 128-column items keep more lanes busy."""
+    columns (two lanes per column) spread each window's row scatter and barriers over
+    twice the columns; in a triangle over fewer than 384 vectors most of them would be
+    half empty, and 128-column items keep more lanes busy.  Where windows are sparse they
+    pay from there on (512 vectors, K = 7: 131 ms, 166 with 128 columns); at K = 5 and 6
+    they do not (77 against 63, 137 against 131; 1,024 vectors 515 against 499).  They stay
+    because two lanes per column make other FP32 runs than four: C would change by 1e-9.
+    A caller free to choose has EngineConfig.tile_cols and autotune()."""
     return 256 if n_cols >= 384 else 128
 
 
