@@ -71,10 +71,10 @@ WORKLOAD_TEXTS = {
 # (profiles/ncu_pair_kernel_counters_fullsize.md gives the commands and figures).  Keyed by
 # (kernel, workload, K, window shift); a launch of anything else reports null.
 PAIR_KERNEL_COUNTERS = {
-    ("k_allpairs<512,1,4>", "uneven1024", 6, 11): {"dram_bytes": 919_221_118_976,
-                                                   "smem_wavefronts": 112_535_121_477},
-    ("k_allpairs<512,1,4>", "uniform256", 6, 11): {"dram_bytes": 41_123_564_544,
-                                                   "smem_wavefronts": 6_131_859_733},
+    ("k_allpairs<512,1,4>", "uneven1024", 6, 11): {"dram_bytes": 919_368_215_296,
+                                                   "smem_wavefronts": 112_216_060_996},
+    ("k_allpairs<512,1,4>", "uniform256", 6, 11): {"dram_bytes": 41_126_181_120,
+                                                   "smem_wavefronts": 6_109_713_934},
 }
 
 
