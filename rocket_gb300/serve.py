@@ -195,7 +195,7 @@ class ServingEngine:
         self.threads: List[threading.Thread] = []
         self.slots: List[_Slot] = []
         self.tuned: Optional[dict] = None
-        self.grid = 1  # CTAs of the pair kernel, once a database is loaded
+        self.grid = 0  # CTAs of the pair kernel, once an engine was made
 
     # -- database -----------------------------------------------------------
     def load(self, proteomes: Proteomes, capacity_vectors: Optional[int] = None,
@@ -296,6 +296,8 @@ class ServingEngine:
                                                  min(nq, self.max_batch), int(cand)))
         staged = float(np.sum(8 * lens + 64)) * 8.0
         roff = nq * (self.db.R + 1) * 4.0
+        if not self.grid:
+            self.grid = PairEngine(self.db.arena, self.cfg).grid
         blocks = fixed_blocks(self.cfg, self.db.R, self.grid, nq, self.db.arena.nnz[:db_n])
         parts = blocks * self.cfg.tile_rows * self.cfg.tile_cols * 8.0
         out = nq * max(db_n, 1) * 8.0

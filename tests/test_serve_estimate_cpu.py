@@ -38,3 +38,15 @@ def test_estimate_reserves_the_plans_blocks(monkeypatch):
     # 64 x 2,048 vectors at K = 7, 1,024 uncut items of 16 x 128 pairs: 17 MB
     assert 1024 * 16 * 128 * 8 <= blocks <= 4 * 1024 * 16 * 128 * 8
     assert srv._estimate(reqs, 0) < with_blocks  # an empty database
+
+
+def test_estimate_asks_an_engine_for_the_grid(monkeypatch):
+    """A database that was not made by load(): the CTAs are those of an engine over it."""
+    srv = ServingEngine("protein", 7, slots=1, cfg=EngineConfig(segments=16))
+    srv.db = SimpleNamespace(R=879440, arena=SimpleNamespace(nnz=_nnz(300)))
+    made = []
+    monkeypatch.setattr(serve, "PairEngine",
+                        lambda arena, cfg: made.append(arena) or SimpleNamespace(grid=GRID))
+    reqs = [Request(0, SimpleNamespace(lengths=lambda: np.full(3, 10 ** 6)))]
+    first = srv._estimate(reqs, 300)
+    assert srv.grid == GRID and first == srv._estimate(reqs, 300) and made == [srv.db.arena]
