@@ -36,3 +36,24 @@ def test_cut_fixed_segments_form_the_whole_ones_sums(monkeypatch, alphabet, k, n
     eng.run(plan, outs[1])
     d = float((outs[0] - outs[1]).abs().max())
     assert d <= TOL, d
+
+
+@pytest.mark.parametrize("rows", [1, 4, 5, 8, 24])
+def test_whole_segments_of_few_rows(rows):
+    """Columns that fill the GPU uncut: whole segments through the kernels of few rows have the
+    bits of whole items."""
+    db = _arena("protein", 5, 300, 0.01)
+    queries = _arena("protein", 5, rows, 0.05)
+    cfg = EngineConfig(segments=64, compress=False)
+    PairEngine(db, cfg).ensure_index()
+    eng = PairEngine(queries, cfg)
+    eng.ensure_index()
+    plan = eng.plan_rect(np.arange(rows), np.arange(300), ldc=300, col_arena=db)
+    assert plan.host_parts is not None and plan.nparts == plan.nitems
+    outs = []
+    for parts in (plan.host_parts, None):
+        plan.host_parts = parts
+        out = torch.full((rows, 300), np.nan, dtype=torch.float64, device="cuda")
+        eng.run(plan, out, diagonal=False, col_arena=db)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all())
